@@ -27,7 +27,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # (__fma_rn / __fmaf_rn); nothing else may be contracted, so the device
 # arithmetic is reproducible bit for bit by the CPU restatement.
 BASE = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(ROOT / "include")]
-CHR_THREADS = (32, 64, 128, 256, 448, 512, 992)
+CHR_THREADS = (32, 64, 128, 256, 512, 992)
+SCREEN_THREADS = (32, 64, 128, 192, 256, 448, 512)
 
 
 def _units():
@@ -35,6 +36,9 @@ def _units():
     for real in ("float", "double"):
         for nt in CHR_THREADS:
             units.append((f"chr_{real}_{nt}", CSRC / "chr_inst.cu",
+                          ["-fmad=false", f"-DNAJA_CHR_REAL={real}", f"-DNAJA_CHR_NT={nt}"]))
+        for nt in SCREEN_THREADS:
+            units.append((f"chr_screen_{real}_{nt}", CSRC / "chr_screen_inst.cu",
                           ["-fmad=false", f"-DNAJA_CHR_REAL={real}", f"-DNAJA_CHR_NT={nt}"]))
     for nt in (128, 256, 512):
         units.append((f"chr_batched_{nt}", CSRC / "chr_batched_inst.cu", ["-fmad=false", f"-DNAJA_CHR_NT={nt}"]))

@@ -73,7 +73,7 @@ DeviceGuard::~DeviceGuard() {
 namespace {
 
 __global__ void pad_convert_kernel(const double* __restrict__ src, long long lds, double* __restrict__ A64,
-                                   float* __restrict__ A32, int m, int d, int lda) {
+                                   float* __restrict__ A32, int m, int d, int lda, int* wide) {
   const long long n = static_cast<long long>(lda) * d;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -82,7 +82,13 @@ __global__ void pad_convert_kernel(const double* __restrict__ src, long long lds
     const double v = (r < m) ? src[c * lds + r] : 0.0;
     A64[i] = v;
     A32[i] = __double2float_rn(v);
+    if (!(fabs(v) <= kScreenMaxA)) *wide = 1;
   }
+}
+
+__global__ void check_rhs_kernel(const double* b, int m, int* wide) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < m && !(fabs(b[r]) <= kScreenMaxB)) *wide = 1;
 }
 
 constexpr unsigned long long kWaitTimeoutNs = 5ull * 1000ull * 1000ull * 1000ull;
@@ -170,6 +176,7 @@ struct naja_polytope {
   float* A32 = nullptr;
   double* b = nullptr;
   int* err = nullptr;
+  bool screen_ok = false;  // |A| <= kScreenMaxA and |b| <= kScreenMaxB everywhere
   std::mutex sparse_mu;
   SparseStore sp;
 };
@@ -403,7 +410,8 @@ int choose_kernel(const naja_polytope* P, const naja_chr_params* p, ChrLaunchCon
                             std::to_string(P->d) + ") does not fit in shared memory");
     }
   }
-  st = chr_plan(p->precision, P->m, P->d, P->lda, p->tpb, p->max_slots, p->nchains, cluster_req, sms, cfg);
+  st = chr_plan(p->precision, P->m, P->d, P->lda, p->tpb, p->max_slots, p->nchains, cluster_req, sms,
+                p->ksparse_prob <= 0.0 && P->screen_ok, cfg);
   if (st == NAJA_ERR_INVALID_ARGUMENT) return fail(st, "Invalid threads per block");
   if (st) return fail(st, "CoordinateHitAndRun: shape (m=" + std::to_string(P->m) + ", d=" + std::to_string(P->d) +
                               ") exceeds the step kernel's capacity for this thread count");
@@ -464,14 +472,22 @@ int naja_polytope_create(int device, int m, int d, const double* A, int lda, con
       e = cudaMemcpy(staged, A, static_cast<size_t>(lda) * d * sizeof(double), cudaMemcpyHostToDevice);
     src = staged;
   }
+  if (e == cudaSuccess) e = cudaMemset(P->err, 0, 4 * sizeof(int));
   if (e == cudaSuccess) {
     const long long total = static_cast<long long>(P->lda) * d;
     const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 16));
-    pad_convert_kernel<<<blocks, 256>>>(src, lda, P->A64, P->A32, m, d, P->lda);
+    pad_convert_kernel<<<blocks, 256>>>(src, lda, P->A64, P->A32, m, d, P->lda, P->err);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)
     e = cudaMemcpy(P->b, b, m * sizeof(double), is_device_ptr(b) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    check_rhs_kernel<<<(m + 255) / 256, 256>>>(P->b, m, P->err);
+    e = cudaGetLastError();
+  }
+  int wide = 0;
+  if (e == cudaSuccess) e = cudaMemcpy(&wide, P->err, sizeof(int), cudaMemcpyDeviceToHost);
+  P->screen_ok = wide == 0;
   if (e == cudaSuccess) e = cudaMemset(P->err, 0, 4 * sizeof(int));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (staged) cudaFree(staged);
@@ -644,6 +660,14 @@ int naja_chr_run(const naja_polytope* P, const naja_chr_params* p, const double*
   a.wait_cycles = p->wait_cycles;
   a.slack_final = dsf;
 
+  // the screened kernel takes its MRG32k3a streams as seeded states
+  DeviceBuffer brs;
+  if (cfg.screen && p->rng == NAJA_RNG_REF_MRG && !p->rng_state) {
+    if ((st = brs.alloc(static_cast<size_t>(p->nchains) * mrg_state_bytes(), stream))) return st;
+    if ((st = mrg_init_states(p->seed, p->chain_base, p->nchains, brs.ptr, stream)))
+      return fail(st, "CoordinateHitAndRun: seeding the MRG32k3a states failed");
+    a.rng_state = brs.ptr;
+  }
   const long long total_steps = static_cast<long long>(p->nspc) * p->thinning;
   const bool segments =
       chr_use_segments(P->m, d, p->resync_interval, total_steps, cfg.cluster, p->wait_cycles != nullptr);

@@ -66,8 +66,8 @@ struct ChrLaunchConfig {
   int slice_lda;  // rows a CTA's column slot holds (cluster > 1), padded to 32
   int max_col;    // sparse-column kernel: entries of the longest compressed column
   int pair_scatter;  // sparse-column kernel: 1 = pair steps through a scratch column, 0 = by search
-  int uniform;       // dense single-CTA kernel: 1 = every warp runs `rows` chunks, the rows past m
-                     // repeating the last V rows (needs m % V == 0); 0 = chunks as rows allow
+  int screen;        // dense single-CTA kernel: 1 = the screened kernel (chr_screen.cuh), `rows` chunks
+                     // per warp exactly; 0 = chr_kernel, `rows` its template capacity
 };
 
 // Compressed columns of A for the sparse-column kernel, in the tier's
@@ -107,8 +107,12 @@ int chr_sparse_launch(int precision, const ChrArgs& args, const SpArgs& sp, int 
 // `cluster`: CTAs per chain, 0 = automatic (one CTA per chain), 1 = one CTA
 // per chain, 2..8 = a thread-block cluster of that many CTAs per chain;
 // `nchains` and `sms` are the launch's chains and the device's SMs.
+// `screen`: the run may take the screened kernel (coordinate and pair steps
+// only, |A| <= kScreenMaxA and |b| <= kScreenMaxB everywhere).
 int chr_plan(int precision, int m, int d, int lda, int tpb, int max_slots, int nchains, int cluster, int sms,
-             ChrLaunchConfig* out);
+             bool screen, ChrLaunchConfig* out);
+constexpr double kScreenMaxA = 288230376151711744.0;             // 2^58
+constexpr double kScreenMaxB = 1267650600228229401496703205376.0;  // 2^100
 
 // Launches nchains independent chains (one CTA each) on `stream`.
 int chr_launch(int precision, const ChrArgs& args, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);

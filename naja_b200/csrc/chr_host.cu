@@ -3,22 +3,27 @@
 
 #include "chr.cuh"
 #include "chr_kernel.cuh"
+#include "chr_screen.cuh"
 
 namespace naja {
 int chr_launch_float_32(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_64(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_128(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_256(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
-int chr_launch_float_448(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_512(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_992(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_32(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_64(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_128(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_256(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
-int chr_launch_double_448(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_512(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_992(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
+
+#define NAJA_SCREEN_DECL(NT)                                                                                       \
+  int chr_screen_launch_float_##NT(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream); \
+  int chr_screen_launch_double_##NT(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
+NAJA_SCREEN_EACH(NAJA_SCREEN_DECL)
+#undef NAJA_SCREEN_DECL
 
 int chr_batch_dispatch_128(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                         const BatchConfig& cfg, cudaStream_t stream, int* occ_out);
@@ -119,9 +124,6 @@ int slack_recompute(const ChrArgs& a, const double* x, int ldx, int nchains, Rea
 // Largest chunks-per-warp capacity used for a thread count (the slack of R
 // chunks takes R * V registers per thread, V rows per lane and chunk).
 int max_chunks_for(int threads, int v) { return (threads <= 512 ? 32 : 16) / v; }
-// Largest chunk count of the uniform-chunk kernels (instantiated 1..8).
-constexpr int kMaxUniformChunks = 8;
-
 }  // namespace
 
 namespace {
@@ -167,24 +169,48 @@ int plan_single(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   out->slice_lda = lda;
   out->max_col = 0;
   out->pair_scatter = 0;
-  out->uniform = 0;
-  // Uniform chunks: every warp runs the same R = ceil(chunks / warps)
-  // chunks as one straight-line row pass (rows past m repeat the last V).
-  const int v = standalone_v(precision), exact = (chunks + warps - 1) / warps;
-  if (m % v == 0 && m >= v && exact <= kMaxUniformChunks && exact <= max_chunks_for(threads, v)) {
-    out->uniform = 1;
-    out->rows = exact;
-    // 14 warps where they hold the same chunks per warp as 16: fewer row
-    // slots repeat (m 5200: 42 for 41 chunks instead of 48); the layout
-    // depends on the thread count, so it is planned again
-    if (tpb <= 0 && threads == 512 && 14 * exact >= chunks) {
-      const Layout L448 = make_layout(d, lda, elt, 448, slots);
-      if (L448.total <= kSmemBudget) {
-        out->threads = 448;
-        out->smem = L448.total;
-      }
+  out->screen = 0;
+  return NAJA_OK;
+}
+
+// The screened kernel, where the rows fit its registers and three columns its
+// shared memory.  Automatic thread count: the fewest threads that hold the
+// rows in at most 5 chunks per warp, up to 192 (FP64 256) threads, then 448.
+// A step's chain of latencies grows with the warps that meet at its barrier,
+// its instructions per warp with the chunks; measured on 16 chains, us per
+// step (FP32): m = 500: 0.498 with 32 threads, 0.532 with 128, 0.592 with
+// 448; m = 1200: 0.540 with 64, 0.594 with 128; m = 2500: 0.663 with 128,
+// 0.701 with 448; m = 5200: 0.969 with 448, 1.057 with 256, 1.227 with 512.
+// FP64: m = 1200: 0.967 with 128, 1.015 with 448; m = 2500: 1.043 with 256,
+// 1.104 with 512; m = 5200: 1.420 with 448, 2.191 with 512 (which spills).
+int plan_screen(int precision, int m, int d, int lda, int tpb, int max_slots, ChrLaunchConfig* out) {
+  const bool f64 = precision == NAJA_PREC_FP64;
+  const int elt = f64 ? 8 : 4;
+  const int chunk = 32 * standalone_v(precision);
+  const int chunks = (m + chunk - 1) / chunk;
+  auto per_warp = [&](int nt) { return (chunks + nt / 32 - 1) / (nt / 32); };
+  int threads = 0;
+  for (const int* t = screen_threads(); *t && !threads; ++t) {
+    if (tpb > 0) {
+      if (*t == tpb) threads = *t;
+    } else if (*t <= (f64 ? 256 : 192) ? per_warp(*t) <= 5 : *t >= 448 && per_warp(*t) <= screen_max_chunks(f64, *t)) {
+      threads = *t;
     }
   }
+  if (!threads || per_warp(threads) > screen_max_chunks(f64, threads)) return NAJA_ERR_UNSUPPORTED;
+  int slots = kMaxSlots;
+  if (max_slots > 0 && max_slots < slots) slots = max_slots;
+  while (slots >= 3 && make_screen_layout(d, lda, elt, threads, slots).total > kSmemBudget) --slots;
+  if (slots < 3) return NAJA_ERR_UNSUPPORTED;
+  out->threads = threads;
+  out->rows = per_warp(threads);
+  out->slots = slots;
+  out->smem = make_screen_layout(d, lda, elt, threads, slots).total;
+  out->cluster = 1;
+  out->slice_lda = lda;
+  out->max_col = 0;
+  out->pair_scatter = 0;
+  out->screen = 1;
   return NAJA_OK;
 }
 
@@ -226,13 +252,13 @@ int plan_cluster(int precision, int m, int d, int tpb, int max_slots, int cs, Ch
   out->slice_lda = slda;
   out->max_col = 0;
   out->pair_scatter = 0;
-  out->uniform = 0;
+  out->screen = 0;
   return NAJA_OK;
 }
 }  // namespace
 
 int chr_plan(int precision, int m, int d, int lda, int tpb, int max_slots, int nchains, int cluster, int sms,
-             ChrLaunchConfig* out) {
+             bool screen, ChrLaunchConfig* out) {
   if (cluster < 0 || cluster > 8) return NAJA_ERR_INVALID_ARGUMENT;
   // Automatic is one CTA per chain: splitting a chain over a cluster was
   // measured slower at every size tried (16 chains, m = 5200: 2.8-6.8 us per
@@ -241,18 +267,29 @@ int chr_plan(int precision, int m, int d, int lda, int tpb, int max_slots, int n
   (void)nchains;
   (void)sms;
   if (cluster >= 2) return plan_cluster(precision, m, d, tpb, max_slots, cluster, out);
+  if (screen && plan_screen(precision, m, d, lda, tpb, max_slots, out) == NAJA_OK) return NAJA_OK;
   return plan_single(precision, m, d, lda, tpb, max_slots, out);
 }
 
 int chr_launch(int precision, const ChrArgs& args, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream) {
   if (nchains <= 0) return NAJA_OK;
   const bool f64 = precision == NAJA_PREC_FP64;
+  if (cfg.screen) {
+#define NAJA_SCREEN_NT(NT)                                                    \
+  case NT:                                                                    \
+    return f64 ? chr_screen_launch_double_##NT(args, nchains, cfg, stream)    \
+               : chr_screen_launch_float_##NT(args, nchains, cfg, stream);
+    switch (cfg.threads) {
+      NAJA_SCREEN_EACH(NAJA_SCREEN_NT)
+      default: return NAJA_ERR_UNSUPPORTED;
+    }
+#undef NAJA_SCREEN_NT
+  }
   switch (cfg.threads) {
     case 32: return f64 ? chr_launch_double_32(args, nchains, cfg, stream) : chr_launch_float_32(args, nchains, cfg, stream);
     case 64: return f64 ? chr_launch_double_64(args, nchains, cfg, stream) : chr_launch_float_64(args, nchains, cfg, stream);
     case 128: return f64 ? chr_launch_double_128(args, nchains, cfg, stream) : chr_launch_float_128(args, nchains, cfg, stream);
     case 256: return f64 ? chr_launch_double_256(args, nchains, cfg, stream) : chr_launch_float_256(args, nchains, cfg, stream);
-    case 448: return f64 ? chr_launch_double_448(args, nchains, cfg, stream) : chr_launch_float_448(args, nchains, cfg, stream);
     case 512: return f64 ? chr_launch_double_512(args, nchains, cfg, stream) : chr_launch_float_512(args, nchains, cfg, stream);
     case 992: return f64 ? chr_launch_double_992(args, nchains, cfg, stream) : chr_launch_float_992(args, nchains, cfg, stream);
     default: return NAJA_ERR_UNSUPPORTED;
