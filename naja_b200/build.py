@@ -40,6 +40,10 @@ def _units():
         for nt in SCREEN_THREADS:
             units.append((f"chr_screen_{real}_{nt}", CSRC / "chr_screen_inst.cu",
                           ["-fmad=false", f"-DNAJA_CHR_REAL={real}", f"-DNAJA_CHR_NT={nt}"]))
+    for real in ("float", "double"):
+        for nw in (1, 2, 4, 8):
+            units.append((f"chr_columns_{real}_{nw}", CSRC / "chr_columns_inst.cu",
+                          ["-fmad=false", f"-DNAJA_CHR_REAL={real}", f"-DNAJA_CHR_NW={nw}"]))
     for nt in (128, 256, 512):
         units.append((f"chr_batched_{nt}", CSRC / "chr_batched_inst.cu", ["-fmad=false", f"-DNAJA_CHR_NT={nt}"]))
     units.append(("chr_sparse", CSRC / "chr_sparse_inst.cu", ["-fmad=false"]))

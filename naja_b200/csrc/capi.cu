@@ -165,6 +165,12 @@ struct SparseStore {
   void* cols64 = nullptr;   // (double, int, pad) entries of A64 by columns
   int* cs64 = nullptr;
   int max64 = 0;
+  // the columns as chr_columns.cuh reads them, by precision and log2 of the
+  // row warps (built when first asked for); lane_entries 0: not built, -1: a
+  // lane would hold more than 8 entries
+  void* lanes[2][4] = {};
+  int lane_entries[2][4] = {};
+  std::vector<int> row_nnz;  // nonzeros of the FP64 A by rows
   int* row_start = nullptr; // A64 by rows, (value, column) entries in groups of kSpRowGroup
   void* row_ent = nullptr;
 };
@@ -192,6 +198,8 @@ void free_sparse(SparseStore& s) {
   cudaFree(s.cs32);
   cudaFree(s.cols64);
   cudaFree(s.cs64);
+  for (auto& p : s.lanes)
+    for (void* q : p) cudaFree(q);
   cudaFree(s.row_start);
   cudaFree(s.row_ent);
   s = SparseStore();
@@ -281,6 +289,39 @@ __global__ void sp_fill_rows_kernel(const double* A64, int m, int d, int lda, co
   for (int q = p + lane; q < row_start[r + 1]; q += 32) row_ent[q] = SpE64{0.0, 0, 0};
 }
 
+// For each column (a block) and warp w of the row ranges bound[w] .. bound[w +
+// 1], entries of that range: their number (lanes null; the largest one in
+// *most) or the column in lane order, `e` entries per lane.
+template <class E>
+__global__ void sp_lanes_kernel(const E* cols, const int* cs, int m, const int* bound, int nw, int e, E* lanes,
+                                int* most) {
+  const int j = blockIdx.x;
+  const E* c = cols + cs[j];
+  const int n = cs[j + 1] - cs[j];
+  auto below = [&](int r) {  // entries of rows below r (rows ascend)
+    int lo = 0, hi = n;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (c[mid].r < r) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  };
+  for (int w = 0; w < nw; ++w) {
+    const int lo = below(bound[w]), k = below(bound[w + 1]) - lo;
+    if (!lanes) {
+      if (threadIdx.x == 0) atomicMax(most, k);
+      continue;
+    }
+    E* out = lanes + (static_cast<size_t>(j) * nw + w) * e * 32;
+    for (int i = threadIdx.x; i < e * 32; i += blockDim.x) {
+      E none{};
+      none.r = m;
+      out[i] = i < k ? c[lo + i] : none;
+    }
+  }
+}
+
 // Builds the compressed columns of both tiers (entries where the tier's A
 // is nonzero, rows ascending, padded with (0, m) entries to 16 bytes) and
 // the FP64 rows (columns ascending) from the device copies of A: counts on
@@ -348,6 +389,7 @@ int build_sparse(naja_polytope* P) {
     free_sparse(S);
     return fail(NAJA_ERR_NO_MEMORY, std::string("building compressed columns: ") + cudaGetErrorString(e));
   }
+  S.row_nnz.assign(h.begin() + 2 * d, h.end());
   S.max32 = max32;
   S.max64 = max64;
   S.tot32 = t32;
@@ -355,6 +397,59 @@ int build_sparse(naja_polytope* P) {
   S.nnz = nnz;
   S.built = true;
   return NAJA_OK;
+}
+
+// The columns in lane order for 2^k row warps (built compressed columns;
+// the caller holds sparse_mu): the row ranges hold equally many nonzeros.
+template <class E>
+int build_lanes(naja_polytope* P, bool f64, int k, const E* cols, const int* cs) {
+  SparseStore& S = P->sp;
+  const int nw = 1 << k;
+  std::vector<int> bound(nw + 1, P->m);
+  bound[0] = 0;
+  long long seen = 0;
+  for (int r = 0, w = 1; r < P->m && w < nw; ++r) {
+    seen += S.row_nnz[r];
+    while (w < nw && seen * nw >= S.nnz * w) bound[w++] = r + 1;
+  }
+  int* dev = nullptr;  // bounds, then the largest share
+  int most = 0;
+  cudaError_t e = cudaMalloc(&dev, (nw + 2) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(dev, 0, (nw + 2) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemcpy(dev, bound.data(), (nw + 1) * sizeof(int), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    sp_lanes_kernel<E><<<P->d, 32>>>(cols, cs, P->m, dev, nw, 0, nullptr, dev + nw + 1);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(&most, dev + nw + 1, sizeof(int), cudaMemcpyDeviceToHost);
+  int entries = -1;
+  for (int c : {8, 6, 4, 3, 2, 1})
+    if (32 * c >= most) entries = c;
+  void* lanes = nullptr;
+  if (e == cudaSuccess && entries > 0) {
+    e = cudaMalloc(&lanes, static_cast<size_t>(P->d) * nw * entries * 32 * sizeof(E));
+    if (e == cudaSuccess) {
+      sp_lanes_kernel<E><<<P->d, 128>>>(cols, cs, P->m, dev, nw, entries, static_cast<E*>(lanes), nullptr);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
+  cudaFree(dev);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(lanes);
+    return fail(NAJA_ERR_NO_MEMORY, std::string("building compressed columns: ") + cudaGetErrorString(e));
+  }
+  S.lanes[f64][k] = lanes;
+  S.lane_entries[f64][k] = entries;
+  return NAJA_OK;
+}
+
+int ensure_lanes(naja_polytope* P, bool f64, int k) {
+  SparseStore& S = P->sp;
+  if (S.lane_entries[f64][k]) return NAJA_OK;
+  return f64 ? build_lanes(P, f64, k, static_cast<const SpE64*>(S.cols64), S.cs64)
+             : build_lanes(P, f64, k, static_cast<const SpE32*>(S.cols32), S.cs32);
 }
 
 }  // namespace sparse_build
@@ -366,7 +461,7 @@ namespace {
 // average and the chain's state fits on chip.  Results are the same either
 // way.
 int choose_kernel(const naja_polytope* P, const naja_chr_params* p, ChrLaunchConfig* cfg, SpArgs* spa,
-                  bool* use_sparse) {
+                  bool* use_sparse, cudaStream_t stream = nullptr) {
   if (p->cluster < 0 || p->cluster > 8)
     return fail(NAJA_ERR_INVALID_ARGUMENT, "naja_chr_run: cluster must be 0 (automatic) or 1..8");
   if (p->sparse < NAJA_SPARSE_AUTO || p->sparse > NAJA_SPARSE_COLUMNS)
@@ -395,8 +490,21 @@ int choose_kernel(const naja_polytope* P, const naja_chr_params* p, ChrLaunchCon
     const int max_col = f64 ? S.max64 : S.max32;
     const long long tot = f64 ? S.tot64 : S.tot32;
     if (p->sparse == NAJA_SPARSE_COLUMNS || 4 * tot <= static_cast<long long>(P->m) * P->d) {
-      st = chr_sparse_plan(p->precision, P->m, P->d, max_col, static_cast<double>(tot) / P->d, p->tpb,
-                           p->max_slots, cfg);
+      const double mean = static_cast<double>(tot) / P->d;
+      st = NAJA_ERR_UNSUPPORTED;
+      const int nw = P->screen_ok ? chr_columns_warps(mean, p->tpb) : 0;
+      const int k = nw == 8 ? 3 : nw == 4 ? 2 : nw == 2 ? 1 : 0;
+      if (nw > 0) {
+        // (building synchronises: a run under capture before it takes chr_sparse.cuh's kernel)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (!S.lane_entries[f64][k] && stream) cudaStreamIsCapturing(stream, &cap);
+        if (cap == cudaStreamCaptureStatusNone)
+          if (int e = sparse_build::ensure_lanes(Pm, f64, k)) return e;
+        if (S.lane_entries[f64][k] > 0)
+          st = chr_columns_plan(p->precision, P->m, P->d, nw, S.lane_entries[f64][k], p->max_slots, cfg);
+        if (st == NAJA_OK) spa->lanes = S.lanes[f64][k];
+      }
+      if (st) st = chr_sparse_plan(p->precision, P->m, P->d, max_col, mean, p->tpb, p->max_slots, cfg);
       if (st == NAJA_OK) {
         *use_sparse = true;
         spa->cols = f64 ? S.cols64 : S.cols32;
@@ -578,7 +686,7 @@ int naja_chr_run(const naja_polytope* P, const naja_chr_params* p, const double*
   ChrLaunchConfig cfg;
   SpArgs spa;
   bool use_sparse = false;
-  int st = choose_kernel(P, p, &cfg, &spa, &use_sparse);
+  int st = choose_kernel(P, p, &cfg, &spa, &use_sparse, stream);
   if (st) return st;
 
   const int d = P->d;
@@ -660,9 +768,9 @@ int naja_chr_run(const naja_polytope* P, const naja_chr_params* p, const double*
   a.wait_cycles = p->wait_cycles;
   a.slack_final = dsf;
 
-  // the screened kernel takes its MRG32k3a streams as seeded states
+  // the screened and the columns kernel take their MRG32k3a streams as seeded states
   DeviceBuffer brs;
-  if (cfg.screen && p->rng == NAJA_RNG_REF_MRG && !p->rng_state) {
+  if ((cfg.screen || cfg.columns) && p->rng == NAJA_RNG_REF_MRG && !p->rng_state) {
     if ((st = brs.alloc(static_cast<size_t>(p->nchains) * mrg_state_bytes(), stream))) return st;
     if ((st = mrg_init_states(p->seed, p->chain_base, p->nchains, brs.ptr, stream)))
       return fail(st, "CoordinateHitAndRun: seeding the MRG32k3a states failed");

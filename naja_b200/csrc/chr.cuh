@@ -64,7 +64,10 @@ struct ChrLaunchConfig {
   size_t smem;    // dynamic shared memory bytes
   int cluster;    // CTAs per chain (thread-block cluster); 1 = one CTA per chain
   int slice_lda;  // rows a CTA's column slot holds (cluster > 1), padded to 32
-  int max_col;    // sparse-column kernel: entries of the longest compressed column
+  int max_col;    // compressed columns: entries of the longest column
+  int columns;    // compressed columns: 1 = chr_columns.cuh, 0 = chr_sparse.cuh
+  int entries;    // chr_columns.cuh: entries of a column per lane (template capacity)
+  int resident;   // chr_columns.cuh: 1 = all columns stay in shared memory (the ring is not used)
   int pair_scatter;  // sparse-column kernel: 1 = pair steps through a scratch column, 0 = by search
   int screen;        // dense single-CTA kernel: 1 = the screened kernel (chr_screen.cuh), `rows` chunks
                      // per warp exactly; 0 = chr_kernel, `rows` its template capacity
@@ -77,12 +80,16 @@ struct ChrLaunchConfig {
 // FP64 A by rows for the FP64 slack recompute: row r's (value, column)
 // entries (16 bytes each, columns ascending) are row_ent[row_start[r],
 // row_start[r + 1]), padded with (0, 0) entries to a multiple of
-// kSpRowGroup.
+// kSpRowGroup.  lanes holds the columns as chr_columns.cuh reads them: 32 W E
+// entries each (W warps, E entries per lane; entry (w E + k) 32 + l is lane
+// l's k-th one of warp w), (0, m) where a lane has none, every row in the same
+// warp throughout.
 struct SpArgs {
   const void* cols;
   const int* col_start;
   const int* row_start;
   const void* row_ent;
+  const void* lanes;
 };
 constexpr int kSpRowGroup = 16;
 
@@ -97,6 +104,13 @@ constexpr int kSpEntryBytes64 = 16;
 // (NAJA_ERR_UNSUPPORTED when the chain's state does not fit on chip).
 int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, int tpb, int max_slots,
                     ChrLaunchConfig* out);
+// Row warps of chr_columns.cuh's kernel: tpb / 32 when forced (0 where it has
+// none), else from the mean column length.
+int chr_columns_warps(double mean_col, int tpb);
+// Plans it for `nw` row warps and `entries` per lane (1, 2, 3, 4, 6 or 8).
+// NAJA_ERR_UNSUPPORTED where the chain's state does not fit.
+int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, ChrLaunchConfig* out);
+// Launches the kernel cfg plans (columns: chr_columns.cuh, else chr_sparse.cuh).
 int chr_sparse_launch(int precision, const ChrArgs& args, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg,
                       cudaStream_t stream);
 

@@ -169,6 +169,9 @@ int plan_single(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   out->slice_lda = lda;
   out->max_col = 0;
   out->pair_scatter = 0;
+  out->columns = 0;
+  out->entries = 0;
+  out->resident = 0;
   out->screen = 0;
   return NAJA_OK;
 }
@@ -210,6 +213,9 @@ int plan_screen(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   out->slice_lda = lda;
   out->max_col = 0;
   out->pair_scatter = 0;
+  out->columns = 0;
+  out->entries = 0;
+  out->resident = 0;
   out->screen = 1;
   return NAJA_OK;
 }
@@ -252,6 +258,9 @@ int plan_cluster(int precision, int m, int d, int tpb, int max_slots, int cs, Ch
   out->slice_lda = slda;
   out->max_col = 0;
   out->pair_scatter = 0;
+  out->columns = 0;
+  out->entries = 0;
+  out->resident = 0;
   out->screen = 0;
   return NAJA_OK;
 }

@@ -1,8 +1,51 @@
 // Planning and launch of the sparse-column CHR step kernel (chr_sparse.cuh).
-#include "chr_sparse.cuh"
+#include "chr_columns.cuh"
 
 namespace naja {
+#define NAJA_COL_EACH(X) X(1) X(2) X(4) X(8)
+#define NAJA_COL_DECL(NW)                                                                                  \
+  int chr_columns_launch_float_##NW(const ChrArgs& a, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg, \
+                                    cudaStream_t stream);                                                  \
+  int chr_columns_launch_double_##NW(const ChrArgs& a, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg, \
+                                     cudaStream_t stream);
+NAJA_COL_EACH(NAJA_COL_DECL)
+#undef NAJA_COL_DECL
+
 using namespace chr_detail;
+
+int chr_columns_warps(double mean_col, int tpb) {
+  if (tpb > 0) return tpb == 32 || tpb == 64 || tpb == 128 || tpb == 256 ? tpb / 32 : 0;
+  // at most two entries of a mean column per lane (us per step, 16 chains,
+  // FP32 / FP64: 416 entries per column 0.814 / 1.288 with 8 warps, 0.858 /
+  // 1.755 with 4, 0.917 / 2.006 with 2; 200 entries 0.654 / 1.061 with 4; 2
+  // entries 0.388 with 1, 0.546 with 4)
+  int nw = 1;
+  while (nw < 8 && mean_col > 64.0 * nw) nw *= 2;
+  return nw;
+}
+
+int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, ChrLaunchConfig* out) {
+  const int elt = precision == NAJA_PREC_FP64 ? 8 : 4;
+  auto bytes = [&](int slots) { return make_col_layout(d, m, elt, nw, entries, slots).total; };
+  int slots = kMaxSlots;
+  if (max_slots > 0 && max_slots < slots) slots = max_slots;
+  while (slots >= 3 && bytes(slots) > kSmemBudget) --slots;
+  if (slots < 3) return NAJA_ERR_UNSUPPORTED;
+  // all columns in shared memory where they fit beside the chain's state
+  out->resident = nw <= 2 && max_slots <= 0 && bytes(0) <= kSmemBudget;
+  out->threads = nw * 32;
+  out->rows = 0;
+  out->slots = slots;
+  out->smem = bytes(out->resident ? 0 : slots);
+  out->cluster = 1;
+  out->slice_lda = 0;
+  out->max_col = 0;
+  out->columns = 1;
+  out->entries = entries;
+  out->pair_scatter = 0;
+  out->screen = 0;
+  return NAJA_OK;
+}
 
 int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, int tpb, int max_slots,
                     ChrLaunchConfig* out) {
@@ -48,6 +91,9 @@ int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, i
   out->cluster = 1;
   out->slice_lda = 0;
   out->max_col = max_col;
+  out->columns = 0;
+  out->entries = 0;
+  out->resident = 0;
   out->pair_scatter = scatter ? 1 : 0;
   out->screen = 0;
   return NAJA_OK;
@@ -55,6 +101,18 @@ int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, i
 
 int chr_sparse_launch(int precision, const ChrArgs& a, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg,
                       cudaStream_t stream) {
+  if (cfg.columns) {
+    const bool f64 = precision == NAJA_PREC_FP64;
+#define NAJA_COL_LAUNCH(NW)                                                  \
+  case 32 * NW:                                                              \
+    return f64 ? chr_columns_launch_double_##NW(a, sp, nchains, cfg, stream) \
+               : chr_columns_launch_float_##NW(a, sp, nchains, cfg, stream);
+    switch (cfg.threads) {
+      NAJA_COL_EACH(NAJA_COL_LAUNCH)
+      default: return NAJA_ERR_UNSUPPORTED;
+    }
+#undef NAJA_COL_LAUNCH
+  }
   if (precision == NAJA_PREC_FP64) return launch_sparse_nw<double>(a, sp, nchains, cfg, stream);
   return launch_sparse_nw<float>(a, sp, nchains, cfg, stream);
 }
