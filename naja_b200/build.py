@@ -46,6 +46,9 @@ def _units():
                           ["-fmad=false", f"-DNAJA_CHR_REAL={real}", f"-DNAJA_CHR_NW={nw}"]))
     for nt in (128, 256, 512):
         units.append((f"chr_batched_{nt}", CSRC / "chr_batched_inst.cu", ["-fmad=false", f"-DNAJA_CHR_NT={nt}"]))
+    for nw in (2, 4, 8):
+        units.append((f"chr_columns_batched_{nw}", CSRC / "chr_columns_batched_inst.cu",
+                      ["-fmad=false", f"-DNAJA_CHR_NW={nw}"]))
     units.append(("chr_sparse", CSRC / "chr_sparse_inst.cu", ["-fmad=false"]))
     units.append(("chr_host", CSRC / "chr_host.cu", ["-fmad=false"]))
     units.append(("capi", CSRC / "capi.cu", []))

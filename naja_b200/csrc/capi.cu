@@ -165,15 +165,23 @@ struct SparseStore {
   void* cols64 = nullptr;   // (double, int, pad) entries of A64 by columns
   int* cs64 = nullptr;
   int max64 = 0;
-  // the columns as chr_columns.cuh reads them, by precision and log2 of the
-  // row warps (built when first asked for); lane_entries 0: not built, -1: a
-  // lane would hold more than 8 entries
-  void* lanes[2][4] = {};
+  // the columns as chr_columns.cuh reads them, built when first asked for:
+  // the entries per lane that 2^k row warps need, by precision and k (0: not
+  // known yet, -1: more than 8), and the copies made
   int lane_entries[2][4] = {};
+  struct Lanes {
+    bool f64;
+    int k, entries;
+    void* ptr;
+  };
+  std::vector<Lanes> lanes;
   std::vector<int> row_nnz;  // nonzeros of the FP64 A by rows
   int* row_start = nullptr; // A64 by rows, (value, column) entries in groups of kSpRowGroup
   void* row_ent = nullptr;
 };
+
+// The device error word's ints, and ints of scratch behind them (under sparse_mu).
+constexpr int kErrWords = 4, kScratchWords = 12;
 
 struct naja_polytope {
   int device = 0;
@@ -198,8 +206,7 @@ void free_sparse(SparseStore& s) {
   cudaFree(s.cs32);
   cudaFree(s.cols64);
   cudaFree(s.cs64);
-  for (auto& p : s.lanes)
-    for (void* q : p) cudaFree(q);
+  for (auto& l : s.lanes) cudaFree(l.ptr);
   cudaFree(s.row_start);
   cudaFree(s.row_ent);
   s = SparseStore();
@@ -400,9 +407,11 @@ int build_sparse(naja_polytope* P) {
 }
 
 // The columns in lane order for 2^k row warps (built compressed columns;
-// the caller holds sparse_mu): the row ranges hold equally many nonzeros.
+// the caller holds sparse_mu), at least `at_least` entries per lane; the row
+// ranges hold equally many nonzeros.  Fills *out and lane_entries (then *out
+// is null where a lane would need more than 8).
 template <class E>
-int build_lanes(naja_polytope* P, bool f64, int k, const E* cols, const int* cs) {
+int build_lanes(naja_polytope* P, bool f64, int k, int at_least, const E* cols, const int* cs, const void** out) {
   SparseStore& S = P->sp;
   const int nw = 1 << k;
   std::vector<int> bound(nw + 1, P->m);
@@ -412,21 +421,22 @@ int build_lanes(naja_polytope* P, bool f64, int k, const E* cols, const int* cs)
     seen += S.row_nnz[r];
     while (w < nw && seen * nw >= S.nnz * w) bound[w++] = r + 1;
   }
-  int* dev = nullptr;  // bounds, then the largest share
+  int* dev = P->err + kErrWords;  // bounds, then the largest share
   int most = 0;
-  cudaError_t e = cudaMalloc(&dev, (nw + 2) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(dev, 0, (nw + 2) * sizeof(int));
+  cudaError_t e = cudaMemset(dev + nw + 1, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMemcpy(dev, bound.data(), (nw + 1) * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) {
+  if (e == cudaSuccess && !S.lane_entries[f64][k]) {
     sp_lanes_kernel<E><<<P->d, 32>>>(cols, cs, P->m, dev, nw, 0, nullptr, dev + nw + 1);
     e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(&most, dev + nw + 1, sizeof(int), cudaMemcpyDeviceToHost);
+    int need = -1;
+    for (int c : {8, 6, 5, 4, 3, 2, 1})
+      if (32 * c >= most) need = c;
+    if (e == cudaSuccess) S.lane_entries[f64][k] = need;
   }
-  if (e == cudaSuccess) e = cudaMemcpy(&most, dev + nw + 1, sizeof(int), cudaMemcpyDeviceToHost);
-  int entries = -1;
-  for (int c : {8, 6, 4, 3, 2, 1})
-    if (32 * c >= most) entries = c;
+  const int entries = std::max(S.lane_entries[f64][k], at_least);
   void* lanes = nullptr;
-  if (e == cudaSuccess && entries > 0) {
+  if (e == cudaSuccess && S.lane_entries[f64][k] > 0) {
     e = cudaMalloc(&lanes, static_cast<size_t>(P->d) * nw * entries * 32 * sizeof(E));
     if (e == cudaSuccess) {
       sp_lanes_kernel<E><<<P->d, 128>>>(cols, cs, P->m, dev, nw, entries, static_cast<E*>(lanes), nullptr);
@@ -434,22 +444,31 @@ int build_lanes(naja_polytope* P, bool f64, int k, const E* cols, const int* cs)
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
   }
-  cudaFree(dev);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(lanes);
     return fail(NAJA_ERR_NO_MEMORY, std::string("building compressed columns: ") + cudaGetErrorString(e));
   }
-  S.lanes[f64][k] = lanes;
-  S.lane_entries[f64][k] = entries;
+  if (lanes) S.lanes.push_back({f64, k, entries, lanes});
+  *out = lanes;
   return NAJA_OK;
 }
 
-int ensure_lanes(naja_polytope* P, bool f64, int k) {
+// *out: the lane-ordered columns for 2^k row warps with max(at_least, what
+// they need) entries per lane, null where they need more than 8.  may_build
+// false (building synchronises): null too where they are not there yet.
+int ensure_lanes(naja_polytope* P, bool f64, int k, int at_least, bool may_build, const void** out) {
   SparseStore& S = P->sp;
-  if (S.lane_entries[f64][k]) return NAJA_OK;
-  return f64 ? build_lanes(P, f64, k, static_cast<const SpE64*>(S.cols64), S.cs64)
-             : build_lanes(P, f64, k, static_cast<const SpE32*>(S.cols32), S.cs32);
+  *out = nullptr;
+  if (S.lane_entries[f64][k] < 0) return NAJA_OK;
+  for (const auto& l : S.lanes)
+    if (l.f64 == f64 && l.k == k && l.entries == std::max(S.lane_entries[f64][k], at_least)) {
+      *out = l.ptr;
+      return NAJA_OK;
+    }
+  if (!may_build) return NAJA_OK;
+  return f64 ? build_lanes(P, f64, k, at_least, static_cast<const SpE64*>(S.cols64), S.cs64, out)
+             : build_lanes(P, f64, k, at_least, static_cast<const SpE32*>(S.cols32), S.cs32, out);
 }
 
 }  // namespace sparse_build
@@ -495,14 +514,14 @@ int choose_kernel(const naja_polytope* P, const naja_chr_params* p, ChrLaunchCon
       const int nw = P->screen_ok ? chr_columns_warps(mean, p->tpb) : 0;
       const int k = nw == 8 ? 3 : nw == 4 ? 2 : nw == 2 ? 1 : 0;
       if (nw > 0) {
-        // (building synchronises: a run under capture before it takes chr_sparse.cuh's kernel)
+        // (a run under capture before the columns are built takes chr_sparse.cuh's kernel)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (!S.lane_entries[f64][k] && stream) cudaStreamIsCapturing(stream, &cap);
-        if (cap == cudaStreamCaptureStatusNone)
-          if (int e = sparse_build::ensure_lanes(Pm, f64, k)) return e;
-        if (S.lane_entries[f64][k] > 0)
+        if (stream) cudaStreamIsCapturing(stream, &cap);
+        const void* lanes = nullptr;
+        if (int e = sparse_build::ensure_lanes(Pm, f64, k, 0, cap == cudaStreamCaptureStatusNone, &lanes)) return e;
+        if (lanes)
           st = chr_columns_plan(p->precision, P->m, P->d, nw, S.lane_entries[f64][k], p->max_slots, cfg);
-        if (st == NAJA_OK) spa->lanes = S.lanes[f64][k];
+        if (st == NAJA_OK) spa->lanes = lanes;
       }
       if (st) st = chr_sparse_plan(p->precision, P->m, P->d, max_col, mean, p->tpb, p->max_slots, cfg);
       if (st == NAJA_OK) {
@@ -566,7 +585,7 @@ int naja_polytope_create(int device, int m, int d, const double* A, int lda, con
   cudaError_t e = cudaMalloc(&P->A64, n * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&P->A32, n * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&P->b, m * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&P->err, 4 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&P->err, (kErrWords + kScratchWords) * sizeof(int));
   if (e != cudaSuccess) {
     cudaGetLastError();
     naja_polytope_destroy(P);
@@ -848,10 +867,16 @@ struct BatchPrep {
   int device = 0;
 };
 
+// Row warps of a compressed batch as the k of SparseStore::lanes, -1 for none.
+int batch_lane_k(int threads) { return threads == 64 ? 1 : threads == 128 ? 2 : threads == 256 ? 3 : -1; }
+
 // Builds every model's compressed columns (once per polytope) and records
-// the longest FP32 column for a compressed-column batch.
-int batch_sparse_prepare(int nmodels, const naja_polytope* const* models, BatchConfig* cfg) {
-  int max_col = 0;
+// the longest FP32 column for a compressed-column batch, and with `quick` the
+// entries per lane that hold every model's columns (0 where one has too many).
+int batch_sparse_prepare(int nmodels, const naja_polytope* const* models, bool quick, BatchConfig* cfg) {
+  int max_col = 0, entries = 0;
+  const int k2 = batch_lane_k(cfg->threads);
+  quick = quick && k2 >= 0;
   for (int k = 0; k < nmodels; ++k) {
     naja_polytope* Pm = const_cast<naja_polytope*>(models[k]);
     if (!Pm) return fail(NAJA_ERR_INVALID_ARGUMENT, "naja_chr_run_batched: null model");
@@ -860,9 +885,16 @@ int batch_sparse_prepare(int nmodels, const naja_polytope* const* models, BatchC
     int st = NAJA_OK;
     if (!Pm->sp.built && (st = sparse_build::build_sparse(Pm))) return st;
     max_col = std::max(max_col, Pm->sp.max32);
+    if (quick) {
+      const void* lanes = nullptr;
+      if (!Pm->sp.lane_entries[0][k2] && (st = sparse_build::ensure_lanes(Pm, false, k2, 0, true, &lanes))) return st;
+      quick = Pm->sp.lane_entries[0][k2] > 0;
+      entries = std::max(entries, Pm->sp.lane_entries[0][k2]);
+    }
   }
   cfg->sparse = 1;
   cfg->max_col = max_col;
+  cfg->entries = quick ? entries : 0;
   return NAJA_OK;
 }
 
@@ -913,12 +945,14 @@ int prep_batch(int nmodels, const naja_polytope* const* models, const naja_chr_p
   cfg.slack_smem = c->slack_smem;
   cfg.ctas_per_sm = c->ctas_per_sm;
   int st = NAJA_OK;
+  bool quick = p->rng == NAJA_RNG_PHILOX && p->ksparse_prob <= 0.0;
+  for (int k = 0; k < nmodels; ++k) quick = quick && models[k]->screen_ok;
   if (c->sparse) {
     if (p->ksparse_prob > 0.0)
       return fail(NAJA_ERR_UNSUPPORTED, "naja_chr_run_batched: compressed columns need ksparse_prob = 0");
-    if ((st = batch_sparse_prepare(nmodels, models, &cfg))) return st;
+    if ((st = batch_sparse_prepare(nmodels, models, quick, &cfg))) return st;
   }
-  st = chr_batch_plan(m_max, d, lda_max, &cfg);
+  st = chr_batch_plan(m_max, d, lda_max, quick, &cfg);
   if (st == NAJA_ERR_INVALID_ARGUMENT) return fail(st, "naja_chr_run_batched: bad batch configuration");
   if (st) return fail(st, "naja_chr_run_batched: configuration cannot hold models of " + std::to_string(m_max) + " rows");
   ChrArgs& a = out->base;
@@ -965,6 +999,13 @@ int prep_batch(int nmodels, const naja_polytope* const* models, const naja_chr_p
       m.sp.col_start = P->sp.cs32;
       m.sp.row_start = P->sp.row_start;
       m.sp.row_ent = P->sp.row_ent;
+    }
+    if (cfg.sparse && cfg.entries) {
+      naja_polytope* Pm = const_cast<naja_polytope*>(P);
+      std::lock_guard<std::mutex> lock(Pm->sparse_mu);
+      DeviceGuard g(Pm->device);
+      if ((st = sparse_build::ensure_lanes(Pm, false, batch_lane_k(cfg.threads), cfg.entries, true, &m.sp.lanes)))
+        return st;
     }
   }
   // chains of different models interleave, so resident CTAs spread over models
@@ -1042,11 +1083,13 @@ extern "C" int naja_batch_occupancy(int nmodels, const naja_polytope* const* mod
   cfg.slack_smem = c->slack_smem;
   cfg.ctas_per_sm = c->ctas_per_sm;
   *ctas_per_sm = 0;
+  bool quick = true;
+  for (int k = 0; k < nmodels; ++k) quick = quick && models[k]->screen_ok;
   if (c->sparse) {
-    const int st = batch_sparse_prepare(nmodels, models, &cfg);
+    const int st = batch_sparse_prepare(nmodels, models, quick, &cfg);
     if (st) return st;
   }
-  if (chr_batch_plan(m_max, models[0]->d, lda_max, &cfg) != NAJA_OK) return NAJA_OK;
+  if (chr_batch_plan(m_max, models[0]->d, lda_max, quick, &cfg) != NAJA_OK) return NAJA_OK;
   DeviceGuard g(models[0]->device);
   int st = chr_batch_occupancy(cfg, ctas_per_sm);
   if (st) *ctas_per_sm = 0;

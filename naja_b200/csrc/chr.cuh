@@ -107,7 +107,7 @@ int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, i
 // Row warps of chr_columns.cuh's kernel: tpb / 32 when forced (0 where it has
 // none), else from the mean column length.
 int chr_columns_warps(double mean_col, int tpb);
-// Plans it for `nw` row warps and `entries` per lane (1, 2, 3, 4, 6 or 8).
+// Plans it for `nw` row warps and `entries` per lane (1, 2, 3, 4, 5, 6 or 8).
 // NAJA_ERR_UNSUPPORTED where the chain's state does not fit.
 int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, ChrLaunchConfig* out);
 // Launches the kernel cfg plans (columns: chr_columns.cuh, else chr_sparse.cuh).
@@ -195,6 +195,9 @@ struct BatchConfig {
   size_t smem;
   int sparse;       // 1: the compressed-column kernel (threads 64, 128 or 256)
   int max_col;      // compressed: entries of the longest column of any model
+  int screen;       // dense: 1 = the screened kernel (chr_screen.cuh), which keeps the slack in registers
+                    // whatever slack_smem says
+  int entries;      // compressed: entries per lane of chr_columns.cuh's kernel, 0 = chr_sparse.cuh's
 };
 
 // Chunk-per-warp capacities instantiated for the batched kernel, per
@@ -210,11 +213,14 @@ inline const int* batch_chunk_capacities(int threads, bool slack_smem) {
 }
 
 // Validates a batch configuration for models of at most m_max rows and fills
-// rows / smem.  Returns 0 or a naja status code.
-int chr_batch_plan(int m_max, int d, int lda_max, BatchConfig* cfg);
+// rows / smem.  `quick`: the run may take the screened or the private-rows
+// kernel (Philox streams, no k-sparse steps, every model within kScreenMaxA
+// and kScreenMaxB; compressed: cfg->entries set, 0 for none).  Returns 0 or a
+// naja status code.
+int chr_batch_plan(int m_max, int d, int lda_max, bool quick, BatchConfig* cfg);
 // The same for the compressed-column kernel (cfg->sparse = 1, cfg->max_col
 // set), with its dispatch.
-int chr_sparse_batch_plan(int m_max, int d, BatchConfig* cfg);
+int chr_sparse_batch_plan(int m_max, int d, bool quick, BatchConfig* cfg);
 int chr_sparse_batch_dispatch(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                               const BatchConfig& cfg, cudaStream_t stream, int* occ_out);
 // Resident CTAs per SM the configuration allows (occupancy calculator).

@@ -30,7 +30,7 @@ namespace chr_detail {
 namespace {
 
 constexpr int kColBatch = 16;          // steps drawn together
-constexpr int kStepRecs = 2 * kColBatch;
+constexpr int kColRecs = 2 * kColBatch;
 
 struct ColLayout {
   size_t x_off, slot_off, slot_bytes, rec_off, full_off, empty_off, drawn_off, done_off, post_off, red_off, flag_off,
@@ -50,7 +50,7 @@ __host__ __device__ inline ColLayout make_col_layout(int d, int m, int elt, int 
   L.slots = slots;
   off += L.slot_bytes * (slots ? slots : d);
   L.rec_off = off;
-  off += sizeof(StepRec) * kStepRecs;
+  off += sizeof(StepRec) * kColRecs;
   L.full_off = off;
   off += 8 * static_cast<size_t>(slots);
   L.empty_off = off;
@@ -69,8 +69,8 @@ __host__ __device__ inline ColLayout make_col_layout(int d, int m, int elt, int 
   off = align_up(off + 16, 16);
   L.slack_off = off;
   off = align_up(off + static_cast<size_t>(m + 1) * elt, 16);
-  L.idx_off = off;  // pair steps: where column j holds this row (0: nowhere)
-  off = align_up(off + static_cast<size_t>(m + 1) * 2, 16);
+  L.idx_off = off;  // pair steps: where column j holds this row
+  off = align_up(off + static_cast<size_t>(m + 1) * (e <= 6 ? 1 : 2), 16);
   L.total = align_up(off, 128);
   return L;
 }
@@ -151,9 +151,6 @@ struct ColShared {
     return reinterpret_cast<volatile int*>(smem + L.flag_off) + 2;
   }
   __device__ __forceinline__ double* alpha() const { return reinterpret_cast<double*>(smem + L.alpha_off); }
-  __device__ __forceinline__ unsigned short* idx() const {
-    return reinterpret_cast<unsigned short*>(smem + L.idx_off);
-  }
 };
 
 // ------------------------------------------------------------------ producer
@@ -173,7 +170,7 @@ __device__ __noinline__ void run_col_producer(const ChrArgs& a, const SpArgs& sp
   for (long long t0 = 0; t0 < total && !stop; t0 += kColBatch) {
     const int n = total - t0 < kColBatch ? static_cast<int>(total - t0) : kColBatch;
     const long long batch_id = t0 / kColBatch;
-    StepRec* batch = sh.recs() + (t0 & (kStepRecs - 1));
+    StepRec* batch = sh.recs() + (t0 & (kColRecs - 1));
     if constexpr (RES) {
       // the batch two before this one, in the same half, has been stepped
       if (batch_id >= 2) {
@@ -335,15 +332,15 @@ struct ColStep {
 };
 
 // Barriers over the NW row warps and the state warp:
-//   kBarPost   every row warp has posted the step's extremes; the column of
-//              the step after the next one has landed (the state warp arrives
-//              only then);
+//   kBarPost   every row warp has posted the step's extremes; the next column
+//              to load (EARLY: of the step after the next one) has landed (the
+//              state warp arrives only then);
 //   kBarStep   only in a step that is not certain: its alpha is posted;
 //   kBarExact  row warps only, inside such a step;
 //   kBarX      only around a recompute.
 //
 // ----------------------------------------------------------------- state warp
-template <class Real, int NW, bool RES>
+template <class Real, int NW, bool RES, bool EARLY>
 __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout& L, unsigned char* smem,
                                               int chain_local) {
   constexpr int NB = 32 * NW + 32;
@@ -364,7 +361,7 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
     }
     if constexpr (!RES) {
       const unsigned long long w0 = a.wait_cycles ? clock64() : 0ull;
-      const int n = ok && sh.recs()[u & (kStepRecs - 1)].kind == kPair ? 2 : 1;
+      const int n = ok && sh.recs()[u & (kColRecs - 1)].kind == kPair ? 2 : 1;
       for (int k = 0; k < n && ok; ++k) {
         ok = mbar_wait_bounded(&sh.full()[slot], parity, a.timeout_ns);
         if (++slot == S) {
@@ -389,7 +386,7 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
     for (int q = 0; q < 2; ++q) ColKeys<Real>::none().post(sh.post<Real>(q, NW, NW));
   }
   named_bar_sync(kBarPost, NB);  // step 0 can be read
-  if (ok) {
+  if (EARLY && ok) {
     if (total > 1) ok = arrived(1);
     if (!ok && lane == 0) sh.stop()[1] = 1;
     named_bar_sync(kBarPost, NB);  // step 1 can be read
@@ -398,7 +395,8 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
   if (ok) cur.read(sh.recs()[0]);
   for (long long t = 0; t < total && ok; ++t) {
     const int buf = static_cast<int>(t & 1);
-    if (t + 2 < total) ok = arrived(t + 2);
+    constexpr int kAhead = EARLY ? 2 : 1;
+    if (t + kAhead < total) ok = arrived(t + kAhead);
     if (!ok && lane == 0) {
       // the row warps find the step uncertain and then the flag
       sh.stop()[0] = 1;
@@ -424,7 +422,7 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
         xs[cur.ej] = __fma_rn(a64, static_cast<double>(cur.cj), xs[cur.ej]);
       }
     }
-    cur.read(sh.recs()[(t + 1) & (kStepRecs - 1)]);
+    cur.read(sh.recs()[(t + 1) & (kColRecs - 1)]);
     if (RES && (t & (kColBatch - 1)) == kColBatch - 1 && lane == 0) mbar_arrive(sh.done() + ((t / kColBatch) & 1));
     if (thin_ctr == 0) {
       __syncwarp();
@@ -464,7 +462,10 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
 }
 
 // ------------------------------------------------------------------ row warps
-template <class Real, int NW, int E, bool RES>
+// EARLY: the next step's entries are loaded while the extremes travel (twice
+// the registers); otherwise after the step, for several chains per SM, which
+// hide each other's latencies.
+template <class Real, int NW, int E, bool RES, bool EARLY>
 __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp, const ColLayout& L,
                                              unsigned char* smem, int chain_local) {
   using T = Tier<Real>;
@@ -475,7 +476,11 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
   const ColShared sh(smem, L);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   Real* slack = reinterpret_cast<Real*>(smem + L.slack_off);
-  unsigned short* idx = sh.idx();
+  // A row's place (from 1) among its warp's entries of column j of a pair
+  // step, 0 for none, kTaken once column i's entry has taken it.
+  using Idx = typename std::conditional<(E <= 6), unsigned char, unsigned short>::type;
+  constexpr int kTaken = E <= 6 ? 0xff : 0xffff;
+  Idx* idx = reinterpret_cast<Idx*>(smem + L.idx_off);
   const int m = a.m, d = a.d, S = L.slots;
 
   auto recompute = [&]() {
@@ -534,7 +539,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
         const Ent q = cb[at0 + 32 * k];
         nv2[k] = q.v;
         nr2[k] = q.r;
-        if (q.r < m) idx[q.r] = static_cast<unsigned short>(at0 + 32 * k + 1);
+        if (q.r < m) idx[q.r] = static_cast<Idx>(lane + 32 * k + 1);
       }
       __syncwarp();
 #pragma unroll
@@ -543,8 +548,8 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
           const int at = idx[nr1[k]];
           Real w = Real(0);
           if (at) {
-            w = cb[at - 1].v;
-            idx[nr1[k]] = 0xffffu;  // column i's entry takes this row
+            w = cb[at0 - lane + at - 1].v;
+            idx[nr1[k]] = kTaken;
           }
           nv1[k] = T::pair_ae_r(nv1[k], w, o.ci, o.cj);
         }
@@ -553,7 +558,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
 #pragma unroll
       for (int k = 0; k < E; ++k) {
         if (nr2[k] < m) {
-          const bool taken = idx[nr2[k]] == 0xffffu;
+          const bool taken = idx[nr2[k]] == kTaken;
           idx[nr2[k]] = 0;
           nv2[k] = T::pair_ae_r(Real(0), nv2[k], o.ci, o.cj);
           if (taken) {
@@ -587,13 +592,14 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
   cur.read(sh.recs()[0]);
   load(cur);
   take();
-  named_bar_sync(kBarPost, NB);  // step 1 has arrived
-  if (sh.stop()[1]) return;
+  if constexpr (EARLY) {
+    named_bar_sync(kBarPost, NB);  // step 1 has arrived
+    if (sh.stop()[1]) return;
+  }
   for (long long t = 0; t < total; ++t) {
     const int buf = static_cast<int>(t & 1);
     const bool more = t + 1 < total;
-    const StepRec& nrec = sh.recs()[(t + 1) & (kStepRecs - 1)];
-    nxt.read(nrec);
+    if (EARLY) nxt.read(sh.recs()[(t + 1) & (kColRecs - 1)]);
     Real s1[E], s2[E];
 #pragma unroll
     for (int k = 0; k < E; ++k) s1[k] = slack[r1[k]];
@@ -627,7 +633,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
     e.reduce();
     if (lane == 0) e.post(sh.post<Real>(buf, NW, warp));
     // the next step's entries, while the other warps post
-    if (more) load(nxt);
+    if (EARLY && more) load(nxt);
     named_bar_sync(kBarPost, NB);
     e.read(sh.post<Real>(buf, NW, lane <= NW ? lane : NW));  // the state warp's entry counts only when it gave up
     e.reduce();
@@ -722,6 +728,8 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
       }
       __syncwarp();
     }
+    if (!EARLY) nxt.read(sh.recs()[(t + 1) & (kColRecs - 1)]);
+    if (!EARLY && more) load(nxt);
     take();
     cur = nxt;
   }
@@ -768,10 +776,65 @@ __global__ void __launch_bounds__(NW * 32 + 64, 1)
   if (threadIdx.x >= NW * 32 + 32) {
     col_producer_entry<Real, RES>(a, sp, L, smem, blockIdx.x);
   } else if (threadIdx.x >= NW * 32) {
-    run_col_state<Real, NW, RES>(a, L, smem, blockIdx.x);
+    run_col_state<Real, NW, RES, true>(a, L, smem, blockIdx.x);
   } else {
-    run_col_rows<Real, NW, E, RES>(a, sp, L, smem, blockIdx.x);
+    run_col_rows<Real, NW, E, RES, true>(a, sp, L, smem, blockIdx.x);
   }
+}
+
+// Batched multi-model run: the persistent item loop of chr_batched_kernel
+// (one item = one chain of one model) over the kernel above, columns staged.
+// Layout for the largest model, lane order of E entries for every model.
+template <int NW, int E>
+__global__ void __launch_bounds__(NW * 32 + 64, NW >= 8 ? 2 : (NW == 4 ? 4 : 6))
+    chr_batched_columns_kernel(const __grid_constant__ ChrArgs base, const __grid_constant__ ColLayout L,
+                               const ModelDesc* __restrict__ models, const int* __restrict__ item_model,
+                               const int* __restrict__ item_chain, int nitems) {
+  using Real = float;
+  constexpr int NT = NW * 32;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ ChrArgs item_args;
+  __shared__ SpArgs item_sp;
+  const ColShared sh(smem, L);
+  if (threadIdx.x == 0) *sh.abort_flag() = 0;
+  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+    const int ch = item_chain[item];
+    if (threadIdx.x == 0) {
+      item_args = item_arguments(base, models[item_model[item]]);
+      item_sp = models[item_model[item]].sp;
+    }
+    __syncthreads();
+    if (*sh.abort_flag()) break;  // every thread reads it after the barrier
+    col_prologue<Real, NW, false>(item_args, item_sp, L, smem, ch);
+    __syncthreads();
+    if (threadIdx.x >= NT + 32) {
+      col_producer_entry<Real, false>(item_args, item_sp, L, smem, ch);
+    } else if (threadIdx.x >= NT) {
+      run_col_state<Real, NW, false, false>(item_args, L, smem, ch);
+    } else {
+      run_col_rows<Real, NW, E, false, false>(item_args, item_sp, L, smem, ch);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 0; q < L.slots; ++q) {
+        mbar_inval(&sh.full()[q]);
+        mbar_inval(&sh.empty()[q]);
+      }
+      for (int q = 0; q < 2; ++q) {
+        mbar_inval(sh.drawn() + q);
+        mbar_inval(sh.done() + q);
+      }
+    }
+  }
+}
+
+template <int NW, int E>
+int batch_columns_one(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
+                      const BatchConfig& cfg, cudaStream_t stream, int* occ_out) {
+  return batch_run(chr_batched_columns_kernel<NW, E>, NW * 32 + 64, cfg, nitems, occ_out, [&](auto kern, int grid) {
+    const ColLayout L = make_col_layout(base->d, cfg.lda_max, sizeof(float), NW, E, cfg.slots);
+    kern<<<grid, NW * 32 + 64, cfg.smem, stream>>>(*base, L, models, im, ic, nitems);
+  });
 }
 
 }  // namespace

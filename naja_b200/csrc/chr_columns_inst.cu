@@ -34,6 +34,7 @@ int NAJA_CAT3(chr_columns_launch, NAJA_CHR_REAL, NAJA_CHR_NW)(const ChrArgs& a, 
     NAJA_COL_CASE(2)
     NAJA_COL_CASE(3)
     NAJA_COL_CASE(4)
+    NAJA_COL_CASE(5)
     NAJA_COL_CASE(6)
     NAJA_COL_CASE(8)
     default: return NAJA_ERR_UNSUPPORTED;

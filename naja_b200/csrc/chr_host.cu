@@ -384,11 +384,24 @@ int mrg_init_states(unsigned long long seed, int chain_base, int nchains, void* 
   return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
 }
 
-int chr_batch_plan(int m_max, int d, int lda_max, BatchConfig* cfg) {
-  if (cfg->sparse) return chr_sparse_batch_plan(m_max, d, cfg);
+int chr_batch_plan(int m_max, int d, int lda_max, bool quick, BatchConfig* cfg) {
+  if (cfg->sparse) return chr_sparse_batch_plan(m_max, d, quick, cfg);
   const int nt = cfg->threads;
   if (nt != 128 && nt != 256 && nt != 512) return NAJA_ERR_INVALID_ARGUMENT;
   const int chunks = (m_max + 32 * kBatchV - 1) / (32 * kBatchV), warps = nt / 32;
+  // The screened kernel where the slots it would run with, and as many chains
+  // per SM as asked for, fit.
+  cfg->screen = 0;
+  if (quick && cfg->slots >= 3 && cfg->slots <= kMaxSlots && (chunks + warps - 1) / warps <= screen_batch_max_chunks(nt)) {
+    const ScreenLayout L = make_screen_layout(d, lda_max, 4, nt, cfg->slots);
+    if (L.total + align_up(sizeof(ChrArgs), 128) <= kSmemBudget) {
+      cfg->screen = 1;
+      cfg->rows = (chunks + warps - 1) / warps;
+      cfg->lda_max = lda_max;
+      cfg->smem = L.total;
+      return NAJA_OK;
+    }
+  }
   int rows = 0;
   for (const int* c = batch_chunk_capacities(nt, cfg->slack_smem != 0); *c; ++c) {
     if (*c * warps >= chunks) {

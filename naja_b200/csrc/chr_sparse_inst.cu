@@ -117,11 +117,42 @@ int chr_sparse_launch(int precision, const ChrArgs& a, const SpArgs& sp, int nch
   return launch_sparse_nw<float>(a, sp, nchains, cfg, stream);
 }
 
-int chr_sparse_batch_plan(int m_max, int d, BatchConfig* cfg) {
+#define NAJA_COLB_EACH(X) X(2) X(4) X(8)
+#define NAJA_COLB_DECL(NW)                                                                                     \
+  int chr_columns_batch_##NW(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems, \
+                             const BatchConfig& cfg, cudaStream_t stream, int* occ_out);
+NAJA_COLB_EACH(NAJA_COLB_DECL)
+#undef NAJA_COLB_DECL
+
+int chr_sparse_batch_plan(int m_max, int d, bool quick, BatchConfig* cfg) {
   const int nt = cfg->threads;
   if (nt != 64 && nt != 128 && nt != 256) return NAJA_ERR_INVALID_ARGUMENT;
   if (cfg->slots < 3 || cfg->slots > kMaxSlots) return NAJA_ERR_INVALID_ARGUMENT;
   if (cfg->max_col <= 0) return NAJA_ERR_UNSUPPORTED;
+  if (quick && cfg->entries > 0) {
+    // A chain's CTA holds the layout, the item's arguments and 1 KB of the
+    // system's.  A ring shallower than asked for is taken where it lets one
+    // more chain per SM run (a second wave of chains costs as much as the
+    // first).
+    const size_t fixed = align_up(sizeof(ChrArgs) + sizeof(SpArgs), 128) + 1024;
+    auto bytes = [&](int slots) { return make_col_layout(d, m_max, 4, nt / 32, cfg->entries, slots).total; };
+    const int most = nt >= 256 ? 2 : (nt == 128 ? 4 : 6);  // chains per SM the registers allow
+    auto chains = [&](int slots) {
+      const int n = static_cast<int>((kSmemBudget + 1024) / (bytes(slots) + fixed));
+      return n < most ? n : most;
+    };
+    int slots = cfg->slots;
+    for (int q = cfg->slots - 1; q >= 3; --q)
+      if (chains(q) > chains(slots)) slots = q;
+    if (chains(slots) > 0) {
+      cfg->slots = slots;
+      cfg->rows = 0;
+      cfg->lda_max = m_max;
+      cfg->smem = bytes(slots);
+      return NAJA_OK;
+    }
+  }
+  cfg->entries = 0;
   const Layout L = make_sparse_layout(d, m_max, 4, kSpEntryBytes32, cfg->max_col, nt / 32, cfg->slots);
   // the kernel also holds one ChrArgs and one SpArgs in static shared memory
   if (L.total + align_up(sizeof(ChrArgs) + sizeof(SpArgs), 128) > kSmemBudget) return NAJA_ERR_UNSUPPORTED;
@@ -133,6 +164,15 @@ int chr_sparse_batch_plan(int m_max, int d, BatchConfig* cfg) {
 
 int chr_sparse_batch_dispatch(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                               const BatchConfig& cfg, cudaStream_t stream, int* occ_out) {
+  if (cfg.entries) {
+#define NAJA_COLB_CASE(NW) \
+  case 32 * NW: return chr_columns_batch_##NW(base, models, im, ic, nitems, cfg, stream, occ_out);
+    switch (cfg.threads) {
+      NAJA_COLB_EACH(NAJA_COLB_CASE)
+      default: return NAJA_ERR_UNSUPPORTED;
+    }
+#undef NAJA_COLB_CASE
+  }
   switch (cfg.threads) {
     case 64: return batch_sparse_one<2>(base, models, im, ic, nitems, cfg, stream, occ_out);
     case 128: return batch_sparse_one<4>(base, models, im, ic, nitems, cfg, stream, occ_out);
