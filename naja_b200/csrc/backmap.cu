@@ -9,12 +9,13 @@
 // back-transformed file.  In GEMM terms V (N x n) = Y (N x d) T^T (d x n).
 //
 // Modes (NAJA_BACKMAP_*):
-//   FP64    SIMT FP64 tiles (the reference's arithmetic, different
+//   FP64    FP64 tensor-core tiles (the reference's arithmetic, different
 //           summation order than cuBLAS).
 //   BF16X3  / TF32X3: split-precision tensor-core products on tcgen05,
 //           in backmap_tc.cu.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <string>
 
 #include "../../include/naja_chr.h"
@@ -24,69 +25,150 @@ namespace naja {
 
 namespace {
 
-constexpr int kBM = 64;  // samples per CTA tile
-constexpr int kBN = 64;  // outputs (rows of T) per CTA tile
+// The FP64 product on the FP64 tensor cores (mma.sync m16n8k8): a CTA takes a
+// 128 x 64 tile of V, eight warps of 32 x 32 each, and streams 16-deep slices
+// of Y and T through a ring of kStages in shared memory (cp.async), Y in its
+// own type and converted as the fragments are read.  What bounds it is the
+// FP64 pipe: per slice a warp issues 16 products of 1,024 multiply-adds and 48
+// shared-memory reads, whose pitches are free of bank conflicts.  The 4 x 4
+// per thread kernel with scalar shared-memory reads it replaces was bound by
+// those reads.  N 40,000, n = d = 700: 4.30 -> 1.32 ms (9.1 -> 29.8 TFLOP/s of
+// about 37).
+constexpr int kBM = 128;  // samples per CTA tile
+constexpr int kBN = 64;   // outputs (rows of T) per CTA tile
 constexpr int kBK = 16;
+constexpr int kStages = 4;
+constexpr int kYPitch = 20;                         // 8 rows x 4 columns on distinct banks
+constexpr int kTPitch = 68;                         // 4 rows x 4 columns on distinct banks
 
-template <class YT, class VT>
-__global__ void __launch_bounds__(256) backmap_fp64_kernel(int n, int d, long long N, const double* __restrict__ T,
-                                                           int ldt, const double* __restrict__ shift,
-                                                           const YT* __restrict__ Y, VT* __restrict__ V) {
-  __shared__ double Ys[kBK][kBM + 1];
-  __shared__ double Ts[kBK][kBN + 1];
-  const long long s0 = static_cast<long long>(blockIdx.x) * kBM;
-  const int i0 = blockIdx.y * kBN;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-  for (int k0 = 0; k0 < d; k0 += kBK) {
-    for (int e = threadIdx.x; e < kBK * kBM; e += 256) {
-      const int kk = e % kBK, ss = e / kBK;
-      const long long s = s0 + ss;
-      Ys[kk][ss] = (s < N && k0 + kk < d) ? static_cast<double>(Y[s * d + k0 + kk]) : 0.0;
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src, bool ok) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(ok ? BYTES : 0)
+                 : "memory");
+}
+
+// Copies a ROWS x COLS block whose rows are `ld` elements apart, from
+// (row0, col0), rows below `rows` and columns below `cols` (zeros beyond).
+// WIDE: 16-byte pieces (every row 16-byte aligned, cols and col0 multiples of
+// a piece, so a piece is inside or outside as a whole).
+template <class E, int ROWS, int COLS, int PITCH, bool WIDE>
+__device__ __forceinline__ void load_block(E* dst, const E* src, long long ld, long long row0, long long rows, int col0,
+                                           int cols) {
+  constexpr int W = WIDE ? 16 / static_cast<int>(sizeof(E)) : 1, PER = COLS / W;
+  for (int e = threadIdx.x; e < ROWS * PER; e += 256) {
+    const int r = e / PER, c = e % PER * W;
+    const bool ok = row0 + r < rows && col0 + c < cols;
+    copy_async<W * static_cast<int>(sizeof(E))>(dst + r * PITCH + c, ok ? src + (row0 + r) * ld + col0 + c : src, ok);
+  }
+}
+
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+template <class YT>
+constexpr size_t fp64_smem_bytes() {
+  return kStages * (kBM * kYPitch * sizeof(YT) + kBK * kTPitch * sizeof(double));
+}
+
+template <class YT, class VT, bool WIDE>
+__global__ void __launch_bounds__(256, 2) backmap_fp64_kernel(int n, int d, long long N, const double* __restrict__ T,
+                                                              int ldt, const double* __restrict__ shift,
+                                                              const YT* __restrict__ Y, VT* __restrict__ V) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  constexpr int YP = kYPitch;
+  YT* ys = reinterpret_cast<YT*>(sm);
+  double* ts = reinterpret_cast<double*>(sm + kStages * kBM * YP * sizeof(YT));
+  const long long s0 = static_cast<long long>(blockIdx.y) * kBM + static_cast<long long>(blockIdx.z) * 65535 * kBM;
+  const int i0 = blockIdx.x * kBN;
+  if (s0 >= N) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
+  const int slices = (d + kBK - 1) / kBK;
+  auto fetch = [&](int k) {
+    if (k < slices) {
+      const int st = k % kStages;
+      load_block<YT, kBM, kBK, YP, WIDE>(ys + st * kBM * YP, Y, d, s0, N, k * kBK, d);
+      load_block<double, kBK, kBN, kTPitch, WIDE>(ts + st * kBK * kTPitch, T, ldt, k * kBK, d, i0, n);
     }
-    for (int e = threadIdx.x; e < kBK * kBN; e += 256) {
-      const int ii = e % kBN, kk = e / kBN;
-      const int i = i0 + ii;
-      Ts[kk][ii] = (i < n && k0 + kk < d) ? T[static_cast<long long>(k0 + kk) * ldt + i] : 0.0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int k = 0; k < kStages - 1; ++k) fetch(k);
+  double acc[2][4][4];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.0;
+  for (int k = 0; k < slices; ++k) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();  // slice k has landed, and everyone is done with the one fetched over next
+    fetch(k + kStages - 1);
+    const YT* yt = ys + k % kStages * kBM * YP;
+    const double* tt = ts + k % kStages * kBK * kTPitch;
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 8) {
+      double a[2][4], b[4][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          a[i][r] = static_cast<double>(yt[(wm + i * 16 + g + (r & 1) * 8) * YP + kk + q + (r >> 1) * 4]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) b[j][r] = tt[(kk + q + r * 4) * kTPitch + wn + j * 8 + g];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma(acc[i][j], a[i], b[j]);
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      double yv[4], tv[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) yv[a] = Ys[kk][ty * 4 + a];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) tv[b] = Ts[kk][tx * 4 + b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = __fma_rn(yv[a], tv[b], acc[a][b]);
-    }
-    __syncthreads();
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const long long s = s0 + ty * 4 + a;
-    if (s >= N) continue;
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int i = i0 + tx * 4 + b;
-      if (i < n) V[s * n + i] = static_cast<VT>(acc[a][b] + shift[i]);
+    for (int h = 0; h < 2; ++h) {
+      const long long s = s0 + wm + i * 16 + g + h * 8;
+      if (s >= N) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int o = i0 + wn + j * 8 + q * 2 + c;
+          if (o < n) V[s * n + o] = static_cast<VT>(acc[i][j][2 * h + c] + shift[o]);
+        }
     }
-  }
+}
+
+template <class YT, class VT, bool WIDE>
+int launch_fp64_as(int n, int d, long long N, const double* T, int ldt, const double* shift, const void* Y, void* V,
+                   cudaStream_t stream) {
+  auto kern = backmap_fp64_kernel<YT, VT, WIDE>;
+  constexpr int smem = static_cast<int>(fp64_smem_bytes<YT>());
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return NAJA_ERR_CUDA;
+  // outputs fastest, so that a block of samples stays in L2 across its tiles
+  const long long rows = (N + kBM - 1) / kBM;
+  const dim3 grid(static_cast<unsigned>((n + kBN - 1) / kBN), static_cast<unsigned>(rows < 65535 ? rows : 65535),
+                  static_cast<unsigned>((rows + 65534) / 65535));
+  kern<<<grid, 256, smem, stream>>>(n, d, N, T, ldt, shift, static_cast<const YT*>(Y), static_cast<VT*>(V));
+  return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
 }
 
 template <class YT, class VT>
 int launch_fp64(int n, int d, long long N, const double* T, int ldt, const double* shift, const void* Y, void* V,
                 cudaStream_t stream) {
-  dim3 grid(static_cast<unsigned>((N + kBM - 1) / kBM), static_cast<unsigned>((n + kBN - 1) / kBN));
-  backmap_fp64_kernel<YT, VT><<<grid, 256, 0, stream>>>(n, d, N, T, ldt, shift, static_cast<const YT*>(Y),
-                                                        static_cast<VT*>(V));
-  return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
+  // 16-byte copies where every row of Y and T starts and ends on 16 bytes
+  const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  const bool wide = aligned(Y) && aligned(T) && d * sizeof(YT) % 16 == 0 && ldt % 2 == 0 && n % 2 == 0;
+  return wide ? launch_fp64_as<YT, VT, true>(n, d, N, T, ldt, shift, Y, V, stream)
+              : launch_fp64_as<YT, VT, false>(n, d, N, T, ldt, shift, Y, V, stream);
 }
 
 }  // namespace
