@@ -65,6 +65,7 @@ class _Buffers:
     act_t: list = field(default_factory=list)    # BF16 (out, pad8(B))
     out: object = None
     target: object = None
+    target_host: object = None  # page-locked, (B, n_out)
     g: list = field(default_factory=list)        # FP32 gradient w.r.t. each layer's pre-activation
     g_bf: list = field(default_factory=list)
     g_bf_t: list = field(default_factory=list)
@@ -158,6 +159,19 @@ class RoundingNet:
         check(self.lib.naja_cast_bf16(z.B, n_in, _p(z.X), z.X.shape[1], _p(z.X_bf), z.X_bf.shape[1], _p(z.X_bf_t),
                                       z.X_bf_t.shape[1], self.stream))
 
+    def _load_targets(self, z, T, n_out):
+        """Targets on the host go through a page-locked buffer of the batch
+        size's own (several cores fill it, one asynchronous copy empties it,
+        both while the forward pass runs); every call that uses it ends with
+        the stream synchronised."""
+        t = self.torch
+        T = t.as_tensor(T, dtype=t.float32)
+        if not T.is_cuda and z.target_host is None:
+            z.target_host = t.empty((z.B, n_out), dtype=t.float32, pin_memory=True)
+        if not T.is_cuda:
+            T = z.target_host.copy_(T)
+        z.target[:, :n_out].copy_(T, non_blocking=True)
+
     def predict(self, X):
         """X (B, n_in) -> outputs (B, n_out) as a float32 CUDA tensor."""
         X = np.asarray(X, np.float32) if not hasattr(X, "data_ptr") else X
@@ -174,8 +188,8 @@ class RoundingNet:
         z = self._buffers(B)
         self._load_inputs(z, X)
         n_out = self.dims[-1]
-        z.target[:, :n_out].copy_(t.as_tensor(T, dtype=t.float32, device=self.device))
         self._forward(z)
+        self._load_targets(z, T, n_out)
         z.loss.zero_()
         nl = len(self.layers)
         wt = None if w is None else t.as_tensor(w, dtype=t.float32, device=self.device).contiguous()
