@@ -865,6 +865,11 @@ struct BatchPrep {
   std::vector<ModelDesc> descs;
   std::vector<int> item_model, item_chain;
   int device = 0;
+  // Runs in segments of `resync` steps (one if 0), each from slacks computed
+  // on the whole GPU (chr_batch_slack) instead of chain by chain: the new
+  // kernels on polytopes of at least kSegmentMinCells cells.
+  bool segmented = false;
+  int nchains = 0, m_max = 0;
 };
 
 // Row warps of a compressed batch as the k of SparseStore::lanes, -1 for none.
@@ -979,6 +984,11 @@ int prep_batch(int nmodels, const naja_polytope* const* models, const naja_chr_p
   a.timeout_ns = kWaitTimeoutNs;
   out->cfg = cfg;
   out->device = models[0]->device;
+  out->nchains = p->nchains;
+  out->m_max = m_max;
+  // (x of two chains has to fit in shared memory)
+  out->segmented = (cfg.sparse ? cfg.entries > 0 : cfg.screen > 0) &&
+                   static_cast<long long>(m_max) * d >= kSegmentMinCells && d <= 14000 && nmodels <= 65535;
   out->descs.resize(nmodels);
   for (int k = 0; k < nmodels; ++k) {
     const naja_polytope* P = models[k];
@@ -992,6 +1002,7 @@ int prep_batch(int nmodels, const naja_polytope* const* models, const naja_chr_p
     m.ldx = ldx;
     m.samples = samples[k];
     m.X_final = X_finals ? X_finals[k] : nullptr;
+    m.slack = nullptr;
     m.seed = p->seed + static_cast<unsigned long long>(k) * seed_stride;
     std::memset(&m.sp, 0, sizeof(m.sp));
     if (cfg.sparse) {
@@ -1017,22 +1028,74 @@ int prep_batch(int nmodels, const naja_polytope* const* models, const naja_chr_p
   return NAJA_OK;
 }
 
-size_t batch_bytes(const BatchPrep& b) {
-  return b.descs.size() * sizeof(ModelDesc) + 2 * b.item_model.size() * sizeof(int) + 64;
+// Device memory of a batched run: the descriptors (of a segmented run three
+// sets: the caller's buffers, and the two directions between the position
+// buffers), the work items, and a segmented run's positions and slacks.
+struct BatchBlock {
+  size_t descs[3], model, chain, upload, x[2], slack, total;
+};
+BatchBlock batch_block(const BatchPrep& b) {
+  BatchBlock k;
+  size_t off = 0;
+  auto take = [&](size_t n) {
+    const size_t at = off;
+    off = (off + n + 255) / 256 * 256;
+    return at;
+  };
+  for (size_t& d : k.descs) d = take((b.segmented || &d == k.descs) ? b.descs.size() * sizeof(ModelDesc) : 0);
+  k.model = take(b.item_model.size() * sizeof(int));
+  k.chain = take(b.item_chain.size() * sizeof(int));
+  k.upload = off;
+  const size_t items = b.item_model.size();
+  for (size_t& x : k.x) x = take(b.segmented ? items * b.base.d * sizeof(double) : 0);
+  k.slack = take(b.segmented ? items * b.m_max * sizeof(float) : 0);
+  k.total = off;
+  return k;
 }
 
-void batch_pack(const BatchPrep& b, std::vector<unsigned char>& host, void* dev, const ModelDesc** dm, const int** im,
-                const int** ic) {
-  host.assign(batch_bytes(b), 0);
-  size_t off = 0;
-  std::memcpy(host.data(), b.descs.data(), b.descs.size() * sizeof(ModelDesc));
-  *dm = reinterpret_cast<const ModelDesc*>(static_cast<char*>(dev) + off);
-  off += (b.descs.size() * sizeof(ModelDesc) + 15) / 16 * 16;
-  std::memcpy(host.data() + off, b.item_model.data(), b.item_model.size() * sizeof(int));
-  *im = reinterpret_cast<const int*>(static_cast<char*>(dev) + off);
-  off += b.item_model.size() * sizeof(int);
-  std::memcpy(host.data() + off, b.item_chain.data(), b.item_chain.size() * sizeof(int));
-  *ic = reinterpret_cast<const int*>(static_cast<char*>(dev) + off);
+// The bytes to upload to the block's first `upload` ones.
+std::vector<unsigned char> batch_pack(const BatchPrep& b, const BatchBlock& k, void* dev) {
+  std::vector<unsigned char> host(k.upload, 0);
+  char* base = static_cast<char*>(dev);
+  for (int set = 0; set < (b.segmented ? 3 : 1); ++set) {
+    std::vector<ModelDesc> d = b.descs;
+    if (set) {
+      const size_t per = static_cast<size_t>(b.nchains) * b.base.d;
+      for (size_t q = 0; q < d.size(); ++q) {
+        d[q].X0 = reinterpret_cast<double*>(base + k.x[set - 1]) + q * per;
+        d[q].X_final = reinterpret_cast<double*>(base + k.x[2 - set]) + q * per;
+        d[q].ldx = b.base.d;
+        d[q].slack = reinterpret_cast<float*>(base + k.slack) + q * b.nchains * b.m_max;
+      }
+    }
+    std::memcpy(host.data() + k.descs[set], d.data(), d.size() * sizeof(ModelDesc));
+  }
+  std::memcpy(host.data() + k.model, b.item_model.data(), b.item_model.size() * sizeof(int));
+  std::memcpy(host.data() + k.chain, b.item_chain.data(), b.item_chain.size() * sizeof(int));
+  return host;
+}
+
+// Queues the run's kernels over an uploaded block.
+int batch_enqueue(const BatchPrep& b, const BatchBlock& k, void* dev, cudaStream_t stream) {
+  char* base = static_cast<char*>(dev);
+  const int items = static_cast<int>(b.item_model.size()), nm = static_cast<int>(b.descs.size()), d = b.base.d;
+  const int *im = reinterpret_cast<const int*>(base + k.model), *ic = reinterpret_cast<const int*>(base + k.chain);
+  auto set = [&](int q) { return reinterpret_cast<const ModelDesc*>(base + k.descs[q]); };
+  if (!b.segmented) return chr_batch_launch(b.base, set(0), im, ic, items, b.cfg, stream);
+  const long long total = static_cast<long long>(b.base.nspc) * b.base.thinning;
+  const long long K = b.base.resync > 0 ? b.base.resync : total;
+  int st = chr_batch_copy_x(set(0), set(1), nm, b.nchains, d, false, stream);
+  int s = 0;
+  for (long long t = 0; t < total && !st; t += K, ++s) {
+    ChrArgs a = b.base;
+    a.t_first = t;
+    a.steps = std::min(K, total - t);
+    a.resync = 0;  // the segment's recompute is the one before it
+    st = chr_batch_slack(set(1 + s % 2), nm, b.nchains, b.m_max, d, stream);
+    if (!st) st = chr_batch_launch(a, set(1 + s % 2), im, ic, items, b.cfg, stream);
+  }
+  if (!st) st = chr_batch_copy_x(set(1 + s % 2), set(0), nm, b.nchains, d, true, stream);
+  return st;
 }
 
 struct GraphHandle {
@@ -1053,15 +1116,13 @@ extern "C" int naja_chr_run_batched(int nmodels, const naja_polytope* const* mod
   if (st) return st;
   DeviceGuard g(b.device);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  const BatchBlock k = batch_block(b);
   DeviceBuffer buf;
-  if ((st = buf.alloc(batch_bytes(b), stream))) return st;
-  std::vector<unsigned char> host;
-  const ModelDesc* dm;
-  const int *im, *ic;
-  batch_pack(b, host, buf.ptr, &dm, &im, &ic);
+  if ((st = buf.alloc(k.total, stream))) return st;
+  const std::vector<unsigned char> host = batch_pack(b, k, buf.ptr);
   cudaError_t e = cudaMemcpyAsync(buf.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
   if (e != cudaSuccess) return fail(NAJA_ERR_CUDA, std::string("naja_chr_run_batched: ") + cudaGetErrorString(e));
-  st = chr_batch_launch(b.base, dm, im, ic, static_cast<int>(b.item_model.size()), b.cfg, stream);
+  st = batch_enqueue(b, k, buf.ptr, stream);
   if (st) return fail(st, std::string("naja_chr_run_batched: launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   // the staging copy above is from pageable memory: it has completed when cudaMemcpyAsync returned
   return NAJA_OK;
@@ -1108,16 +1169,14 @@ extern "C" int naja_chr_capture_batched(int nmodels, const naja_polytope* const*
   DeviceGuard g(b.device);
   GraphHandle* h = new GraphHandle();
   h->device = b.device;
-  cudaError_t e = cudaMalloc(&h->dev, batch_bytes(b));
+  const BatchBlock k = batch_block(b);
+  cudaError_t e = cudaMalloc(&h->dev, k.total);
   if (e == cudaSuccess) e = cudaMalloc(&h->err, 4 * sizeof(int));
   if (e != cudaSuccess) {
     naja_graph_destroy(h);
     return fail(NAJA_ERR_NO_MEMORY, std::string("naja_chr_capture_batched: ") + cudaGetErrorString(e));
   }
-  std::vector<unsigned char> host;
-  const ModelDesc* dm;
-  const int *im, *ic;
-  batch_pack(b, host, h->dev, &dm, &im, &ic);
+  const std::vector<unsigned char> host = batch_pack(b, k, h->dev);
   e = cudaMemcpy(h->dev, host.data(), host.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(h->err, 0, 4 * sizeof(int));
   b.base.err = h->err;
@@ -1127,7 +1186,7 @@ extern "C" int naja_chr_capture_batched(int nmodels, const naja_polytope* const*
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed);
   if (e == cudaSuccess) {
-    st = chr_batch_launch(b.base, dm, im, ic, static_cast<int>(b.item_model.size()), b.cfg, s);
+    st = batch_enqueue(b, k, h->dev, s);
     cudaError_t e2 = cudaStreamEndCapture(s, &h->graph);
     if (st == NAJA_OK) e = e2;
   }

@@ -183,7 +183,17 @@ struct ModelDesc {
   double* X_final;   // nullable
   unsigned long long seed;
   SpArgs sp;         // compressed columns (FP32 tier) for the compressed-column batch
+  float* slack;      // nullable: nchains x m, the chains' slack at the launch's first step
 };
+
+// The slack b - A64 x of every chain (at its X0) of every model into the
+// models' `slack` (the step kernel's recompute, bit for bit), A64 read once
+// for all chains of a model.
+int chr_batch_slack(const ModelDesc* models, int nmodels, int nchains, int m_max, int d, cudaStream_t stream);
+// Copies every chain's X0 of `from` to the X0 of `to` (final = false), or to
+// the X_final of `to` where it has one.
+int chr_batch_copy_x(const ModelDesc* from, const ModelDesc* to, int nmodels, int nchains, int d, bool final,
+                     cudaStream_t stream);
 
 struct BatchConfig {
   int threads;      // consumer threads per chain

@@ -121,6 +121,66 @@ int slack_recompute(const ChrArgs& a, const double* x, int ldx, int nchains, Rea
   return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
 }
 
+// As slack_recompute_kernel for the models of a batch (blockIdx.y), CG chains
+// at a time: each value of A64 is loaded once for CG chains, their x
+// interleaved in shared memory (two per 16-byte read).
+constexpr int kBatchSlackJB = 8;
+template <int CG>
+__global__ void __launch_bounds__(128) batch_slack_kernel(const ModelDesc* __restrict__ models, int nchains, int d) {
+  extern __shared__ __align__(16) double xsh2[];  // d x CG
+  const ModelDesc& md = models[blockIdx.y];
+  const int r = blockIdx.x * 128 + threadIdx.x, m = md.m;
+  if (blockIdx.x * 128 >= m) return;
+  const size_t lda = md.lda;
+  const double* Ar = md.A64 + (r < m ? r : m - 1);
+  for (int c0 = 0; c0 < nchains; c0 += CG) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < CG * d; i += 128) {
+      const int c = i / d, j = i - c * d;
+      xsh2[j * CG + c] = md.X0[static_cast<size_t>(min(c0 + c, nchains - 1)) * md.ldx + j];
+    }
+    __syncthreads();
+    double acc[CG];
+#pragma unroll
+    for (int c = 0; c < CG; ++c) acc[c] = 0.0;
+    auto column = [&](int j, double av) {
+      const double2* xj = reinterpret_cast<const double2*>(xsh2 + j * CG);
+#pragma unroll
+      for (int c = 0; c < CG / 2; ++c) {
+        const double2 v = xj[c];
+        acc[2 * c] = __fma_rn(av, v.x, acc[2 * c]);
+        acc[2 * c + 1] = __fma_rn(av, v.y, acc[2 * c + 1]);
+      }
+    };
+    int j = 0;
+    for (; j + kBatchSlackJB <= d; j += kBatchSlackJB) {
+      double av[kBatchSlackJB];
+#pragma unroll
+      for (int u = 0; u < kBatchSlackJB; ++u) av[u] = __ldg(Ar + (j + u) * lda);
+#pragma unroll
+      for (int u = 0; u < kBatchSlackJB; ++u) column(j + u, av[u]);
+    }
+    for (; j < d; ++j) column(j, __ldg(Ar + j * lda));
+    if (r < m) {
+#pragma unroll
+      for (int c = 0; c < CG; ++c)
+        if (c0 + c < nchains)
+          md.slack[static_cast<size_t>(c0 + c) * m + r] = Tier<float>::from64(__dsub_rn(md.b[r], acc[c]));
+    }
+  }
+}
+
+__global__ void batch_copy_x_kernel(const ModelDesc* __restrict__ from, const ModelDesc* __restrict__ to, int nchains,
+                                    int d, bool final) {
+  const ModelDesc &a = from[blockIdx.x], &b = to[blockIdx.x];
+  double* dst = final ? b.X_final : const_cast<double*>(b.X0);
+  if (!dst) return;
+  for (int i = threadIdx.x; i < nchains * d; i += blockDim.x) {
+    const int c = i / d, j = i - c * d;
+    dst[static_cast<size_t>(c) * b.ldx + j] = a.X0[static_cast<size_t>(c) * a.ldx + j];
+  }
+}
+
 // Largest chunks-per-warp capacity used for a thread count (the slack of R
 // chunks takes R * V registers per thread, V rows per lane and chunk).
 int max_chunks_for(int threads, int v) { return (threads <= 512 ? 32 : 16) / v; }
@@ -439,6 +499,26 @@ int chr_batch_launch(const ChrArgs& base, const ModelDesc* models, const int* it
                      int nitems, const BatchConfig& cfg, cudaStream_t stream) {
   if (nitems <= 0) return NAJA_OK;
   return batch_dispatch(&base, models, item_model, item_chain, nitems, cfg, stream, nullptr);
+}
+
+int chr_batch_slack(const ModelDesc* models, int nmodels, int nchains, int m_max, int d, cudaStream_t stream) {
+  const dim3 grid((m_max + 127) / 128, nmodels);
+  auto launch = [&](auto kern, int cg) {
+    const size_t smem = static_cast<size_t>(cg) * d * sizeof(double);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+      return NAJA_ERR_CUDA;
+    kern<<<grid, 128, smem, stream>>>(models, nchains, d);
+    return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
+  };
+  if (nchains > 4 && d <= 1700) return launch(batch_slack_kernel<8>, 8);
+  if (nchains > 2 && d <= 3400) return launch(batch_slack_kernel<4>, 4);
+  return launch(batch_slack_kernel<2>, 2);
+}
+
+int chr_batch_copy_x(const ModelDesc* from, const ModelDesc* to, int nmodels, int nchains, int d, bool final,
+                     cudaStream_t stream) {
+  batch_copy_x_kernel<<<nmodels, 256, 0, stream>>>(from, to, nchains, d, final);
+  return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
 }
 
 size_t mrg_state_bytes() { return sizeof(curandStateMRG32k3a); }
