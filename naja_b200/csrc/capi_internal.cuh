@@ -70,7 +70,8 @@ int backmap_tc_split_T(int n, int d, const double* T, int ldt, void* Th, void* T
 // Splits Y (N rows of d values, y_dtype) into Yh, Yl and launches the GEMM
 // V = Y T^T + shift against the split T; a bounded wait that expires sets
 // err[0..3].  Asynchronous: nothing is read back.
-int backmap_tc_enqueue(int n, int d, long long N, const void* Y, int y_dtype, const void* Th, const void* Tl, void* Yh,
+long long backmap_tc_chunk_rows(long long N, int n, int d, int mode);
+int backmap_tc_enqueue(int n, int d, long long N, long long chunk, const void* Y, int y_dtype, const void* Th, const void* Tl, void* Yh,
                        void* Yl, const double* shift, void* V, int v_dtype, int mode, int* err, cudaStream_t stream);
 // Synchronises `stream` and turns a set error word into NAJA_ERR_DEVICE.
 int backmap_tc_read_error(const int* err, cudaStream_t stream, const char* who);

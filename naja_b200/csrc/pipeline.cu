@@ -152,6 +152,7 @@ extern "C" int naja_chr_run_backmapped(const naja_polytope* P, const naja_chr_pa
   if (!v_dev && ((st = bv0.alloc(chunk_rows * n * velt, stream)) || (st = bv1.alloc(chunk_rows * n * velt, stream))))
     return st;
   if (tc) {
+    // (a shorter last chunk never takes more rows at a time than a whole one)
     const size_t yb = backmap_tc_operand_bytes(static_cast<long long>(chunk_rows), d, mode);
     const size_t tb = backmap_tc_operand_bytes(n, d, mode);
     if ((st = bTh.alloc(tb, stream)) || (st = bTl.alloc(tb, stream)) || (st = bYh.alloc(yb, stream)) ||
@@ -201,7 +202,7 @@ extern "C" int naja_chr_run_backmapped(const naja_polytope* P, const naja_chr_pa
     const size_t row0 = static_cast<size_t>(k * cs) * nch;
     void* vdst = v_dev ? static_cast<char*>(V) + row0 * n * velt : vbuf[b];
     const void* y = sample_ptr(k);
-    int s2 = tc ? backmap_tc_enqueue(n, d, static_cast<long long>(rows), y, p.out_dtype, bTh.ptr, bTl.ptr, bYh.ptr,
+    int s2 = tc ? backmap_tc_enqueue(n, d, static_cast<long long>(rows), static_cast<long long>(rows), y, p.out_dtype, bTh.ptr, bTl.ptr, bYh.ptr,
                                      bYl.ptr, static_cast<const double*>(dS), vdst, v_dtype, mode,
                                      static_cast<int*>(berr.ptr), ws.bm)
                 : backmap_fp64_enqueue(n, d, static_cast<long long>(rows), static_cast<const double*>(dT), ldt,
