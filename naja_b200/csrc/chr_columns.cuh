@@ -306,38 +306,65 @@ __device__ __noinline__ void col_producer_entry(const ChrArgs& a, const SpArgs& 
   }
 }
 
-// A step's record as the row warps and the state warp read it.
+// The state warp's part of a step: x, and the samples saved from it.
 template <class Real>
-struct ColStep {
-  int kind, ei, ej, flag;
-  Real ci, cj, u;
-  __device__ __forceinline__ void read(const StepRec& r) {
-    const int4 h = *reinterpret_cast<const int4*>(&r.kind);
-    kind = h.x;
-    ei = h.y;
-    ej = h.z;
-    flag = h.w;
-    if constexpr (sizeof(Real) == 4) {
-      const float4 f = *reinterpret_cast<const float4*>(&r.cif);
-      ci = f.x;
-      cj = f.y;
-      u = f.z;
-    } else {
-      const double2 f = *reinterpret_cast<const double2*>(&r.ci);
-      ci = f.x;
-      cj = f.y;
-      u = r.u;
+struct ColMover {
+  const ChrArgs& a;
+  double* xs;
+  const Real* alpha;  // [2]
+  int chain_local, lane, thin_ctr;
+  size_t out_row;
+  ScreenStep<Real> step;
+  __device__ __forceinline__ ColMover(const ChrArgs& a_, double* xs_, const Real* alpha_, int chain_local_, int lane_)
+      : a(a_), xs(xs_), alpha(alpha_), chain_local(chain_local_), lane(lane_) {
+    thin_ctr = static_cast<int>(a.t_first % a.thinning);
+    out_row = static_cast<size_t>(a.chain_base + chain_local) +
+              static_cast<size_t>((a.t_first + a.thinning - 1) / a.thinning) * a.out_nchains;
+  }
+  __device__ __forceinline__ void read(const StepRec& r) { step.read(r); }
+  // Moves x by step t (the record read last), whose alpha is there.
+  __device__ __forceinline__ void move(long long t) {
+    if (lane == 0) {
+      const double a64 = static_cast<double>(*reinterpret_cast<const volatile Real*>(alpha + (t & 1)));
+      if (step.kind == kCoord) {
+        xs[step.ei] = __dadd_rn(xs[step.ei], a64);
+      } else {
+        xs[step.ei] = __fma_rn(a64, static_cast<double>(step.ci), xs[step.ei]);
+        xs[step.ej] = __fma_rn(a64, static_cast<double>(step.cj), xs[step.ej]);
+      }
     }
+    if (thin_ctr == 0) {
+      __syncwarp();
+      const int d = a.d;
+      if (a.samples) {
+        if (a.out_f64) {
+          double* out = reinterpret_cast<double*>(a.samples) + out_row * d;
+          for (int j = lane; j < d; j += 32) out[j] = xs[j];
+        } else {
+          float* out = reinterpret_cast<float*>(a.samples) + out_row * d;
+          for (int j = lane; j < d; j += 32) out[j] = __double2float_rn(xs[j]);
+        }
+      }
+      out_row += static_cast<size_t>(a.out_nchains);
+      __syncwarp();
+    }
+    if (++thin_ctr == a.thinning) thin_ctr = 0;
+  }
+  __device__ __forceinline__ void finish() {
+    __syncwarp();
+    if (a.X_final)
+      for (int j = lane; j < a.d; j += 32) a.X_final[static_cast<size_t>(chain_local) * a.ldx + j] = xs[j];
   }
 };
 
-// Barriers over the NW row warps and the state warp:
-//   kBarPost   every row warp has posted the step's extremes; the next column
-//              to load (EARLY: of the step after the next one) has landed (the
-//              state warp arrives only then);
-//   kBarStep   only in a step that is not certain: its alpha is posted;
-//   kBarExact  row warps only, inside such a step;
-//   kBarX      only around a recompute.
+// Barriers over the NW row warps:
+//   kBarPost   every row warp has posted the step's extremes; with the state
+//              warp, which arrives once the next column to load (EARLY: of the
+//              step after the next one) has landed, and takes up the previous
+//              step's alpha after it;
+//   kBarExact  only inside a step that is not certain;
+//   kBarX      with the state warp, around a recompute (this step's alpha is
+//              there; x has moved; the slack is new) and after the last step.
 //
 // ----------------------------------------------------------------- state warp
 template <class Real, int NW, bool RES, bool EARLY>
@@ -346,7 +373,7 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
   constexpr int NB = 32 * NW + 32;
   const ColShared sh(smem, L);
   const int lane = threadIdx.x & 31;
-  const int d = a.d, S = L.slots;
+  const int S = L.slots;
   double* xs = sh.xs();
   const long long total = launch_steps(a);
   int slot = 0;
@@ -375,13 +402,11 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
     if (!ok && lane == 0) set_error(a.err, kDevTimeoutFull, slot, static_cast<int>(parity), static_cast<int>(u));
     return ok;
   };
-  int thin_ctr = static_cast<int>(a.t_first % a.thinning);
+  ColMover<Real> mover(a, xs, reinterpret_cast<const Real*>(sh.alpha()), chain_local, lane);
   int resync_ctr = a.resync > 0 ? static_cast<int>((a.t_first + 1) % a.resync) : 0;
-  size_t out_row = static_cast<size_t>(a.chain_base + chain_local) +
-                   static_cast<size_t>((a.t_first + a.thinning - 1) / a.thinning) * a.out_nchains;
   bool ok = arrived(0);
   if (lane == 0) {
-    sh.stop()[0] = ok ? 0 : 1;
+    sh.stop()[0] = ok ? -1 : 0;
     sh.stop()[1] = 0;
     for (int q = 0; q < 2; ++q) ColKeys<Real>::none().post(sh.post<Real>(q, NW, NW));
   }
@@ -391,58 +416,32 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
     if (!ok && lane == 0) sh.stop()[1] = 1;
     named_bar_sync(kBarPost, NB);  // step 1 can be read
   }
-  ColStep<Real> cur;
-  if (ok) cur.read(sh.recs()[0]);
+  bool pending = false;  // step t - 1 has not moved x yet
   for (long long t = 0; t < total && ok; ++t) {
-    const int buf = static_cast<int>(t & 1);
     constexpr int kAhead = EARLY ? 2 : 1;
     if (t + kAhead < total) ok = arrived(t + kAhead);
     if (!ok && lane == 0) {
       // the row warps find the step uncertain and then the flag
-      sh.stop()[0] = 1;
-      ColKeys<Real>::nan().post(sh.post<Real>(buf, NW, NW));
+      sh.stop()[0] = static_cast<int>(t & 0x7fffffff);
+      ColKeys<Real>::nan().post(sh.post<Real>(static_cast<int>(t & 1), NW, NW));
     }
     named_bar_sync(kBarPost, NB);
     if (!ok) break;
-    ColKeys<Real> e;
-    e.read(sh.post<Real>(buf, NW, lane < NW ? lane : 0));
-    e.reduce();
-    double a64;
-    if (e.certain() && cur.flag == 0) {
-      a64 = static_cast<double>(e.alpha(cur.u));
-    } else {
-      named_bar_sync(kBarStep, NB);
-      a64 = *sh.alpha();
-    }
-    if (lane == 0) {
-      if (cur.kind == kCoord) {
-        xs[cur.ei] = __dadd_rn(xs[cur.ei], a64);
-      } else {
-        xs[cur.ei] = __fma_rn(a64, static_cast<double>(cur.ci), xs[cur.ei]);
-        xs[cur.ej] = __fma_rn(a64, static_cast<double>(cur.cj), xs[cur.ej]);
-      }
-    }
-    cur.read(sh.recs()[(t + 1) & (kColRecs - 1)]);
-    if (RES && (t & (kColBatch - 1)) == kColBatch - 1 && lane == 0) mbar_arrive(sh.done() + ((t / kColBatch) & 1));
-    if (thin_ctr == 0) {
+    if (pending) mover.move(t - 1);
+    mover.read(sh.recs()[t & (kColRecs - 1)]);
+    // (a half of the records is free once its last one has been read)
+    if (RES && (t & (kColBatch - 1)) == kColBatch - 1) {
       __syncwarp();
-      if (a.samples) {
-        if (a.out_f64) {
-          double* out = reinterpret_cast<double*>(a.samples) + out_row * d;
-          for (int j = lane; j < d; j += 32) out[j] = xs[j];
-        } else {
-          float* out = reinterpret_cast<float*>(a.samples) + out_row * d;
-          for (int j = lane; j < d; j += 32) out[j] = __double2float_rn(xs[j]);
-        }
-      }
-      out_row += static_cast<size_t>(a.out_nchains);
-      __syncwarp();
+      if (lane == 0) mbar_arrive(sh.done() + ((t / kColBatch) & 1));
     }
-    if (++thin_ctr == a.thinning) thin_ctr = 0;
+    pending = true;
     if (a.resync > 0 && t + 1 < total) {
       if (resync_ctr == 0) {
-        named_bar_sync(kBarX, NB);  // x has moved
-        named_bar_sync(kBarX, NB);  // the slack is new
+        named_bar_sync(kBarX, NB);
+        mover.move(t);
+        pending = false;
+        named_bar_sync(kBarX, NB);
+        named_bar_sync(kBarX, NB);
       }
       if (++resync_ctr == a.resync) resync_ctr = 0;
     }
@@ -451,10 +450,9 @@ __device__ __forceinline__ void run_col_state(const ChrArgs& a, const ColLayout&
     *sh.abort_flag() = 1;
     return;
   }
-  __syncwarp();
-  if (a.X_final) {
-    for (int j = lane; j < d; j += 32) a.X_final[static_cast<size_t>(chain_local) * a.ldx + j] = xs[j];
-  }
+  named_bar_sync(kBarX, NB);
+  if (pending) mover.move(total - 1);
+  mover.finish();
   if (a.wait_cycles && lane == 0) {
     a.wait_cycles[4 * chain_local + 0] = w_full;
     a.wait_cycles[4 * chain_local + 2] = clock64() - c_start;
@@ -481,7 +479,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
   using Idx = typename std::conditional<(E <= 6), unsigned char, unsigned short>::type;
   constexpr int kTaken = E <= 6 ? 0xff : 0xffff;
   Idx* idx = reinterpret_cast<Idx*>(smem + L.idx_off);
-  const int m = a.m, d = a.d, S = L.slots;
+  const int m = a.m, S = L.slots;
 
   auto recompute = [&]() {
     const R64* rows = static_cast<const R64*>(sp.row_ent);
@@ -522,7 +520,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
     return c;
   };
   // Loads (and merges) a step's entries into nv / nr and gives its slots back.
-  auto load = [&](const ColStep<Real>& o) {
+  auto load = [&](const ScreenStep<Real>& o) {
     const int sa = slot;
     const Ent* ca = column(o.ei);
 #pragma unroll
@@ -586,9 +584,9 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
 
   const long long total = launch_steps(a);
   int resync_ctr = a.resync > 0 ? static_cast<int>((a.t_first + 1) % a.resync) : 0;
-  ColStep<Real> cur, nxt;
+  ScreenStep<Real> cur, nxt;
   named_bar_sync(kBarPost, NB);  // step 0 has arrived
-  if (sh.stop()[0]) return;
+  if (sh.stop()[0] >= 0) return;
   cur.read(sh.recs()[0]);
   load(cur);
   take();
@@ -635,13 +633,17 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
     // the next step's entries, while the other warps post
     if (EARLY && more) load(nxt);
     named_bar_sync(kBarPost, NB);
-    e.read(sh.post<Real>(buf, NW, lane <= NW ? lane : NW));  // the state warp's entry counts only when it gave up
-    e.reduce();
+    if constexpr (NW > 1) {
+      e.read(sh.post<Real>(buf, NW, lane <= NW ? lane : NW));  // the state warp's entry counts only when it gave up
+      e.reduce();
+    } else {
+      if (sh.stop()[0] >= 0) return;
+    }
     Real alpha;
     if (e.certain() && cur.flag == 0) {
       alpha = e.alpha(cur.u);
     } else {
-      if (sh.stop()[0]) return;
+      if (sh.stop()[0] == static_cast<int>(t & 0x7fffffff)) return;
       // exactly: this step's entries, then, if an end is missing, all rows
       Acc h, l, l2;
       auto block = [&]() {
@@ -707,15 +709,17 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
         T::decode(h, l, l2, mx, mn);
       }
       alpha = T::alpha(mx, mn, cur.u);
-      if (tid == 0) *sh.alpha() = static_cast<double>(alpha);
-      named_bar_sync(kBarStep, NB);
+      // (a dense pass of another warp may still be reading this one's rows)
+      if constexpr (NW > 1) named_bar_sync(kBarExact, NT);
     }
+    if (tid == 0) reinterpret_cast<volatile Real*>(sh.alpha())[buf] = alpha;
     bool again = false;
     if (a.resync > 0 && more) {
       again = resync_ctr == 0;
       if (++resync_ctr == a.resync) resync_ctr = 0;
     }
     if (again) {
+      named_bar_sync(kBarX, NB);
       named_bar_sync(kBarX, NB);  // the state warp has moved x
       recompute();
       named_bar_sync(kBarX, NB);
@@ -733,6 +737,7 @@ __device__ __forceinline__ void run_col_rows(const ChrArgs& a, const SpArgs& sp,
     take();
     cur = nxt;
   }
+  named_bar_sync(kBarX, NB);
   if (a.slack_final) {
     named_bar_sync(kBarExact, NT);
     Real* so = static_cast<Real*>(a.slack_final) + static_cast<size_t>(chain_local) * m;
