@@ -22,7 +22,7 @@
 //                        so that a store covers 32 columns of a row, the
 //                        transposed one is written as the lanes hold it.
 // One training step (2600-512-512-23100, batch 64): the nine products took
-// 480 us with 128 x 128 tiles and a row per thread in the stores, 210 us now.
+// 480 us with 128 x 128 tiles and a row per thread in the stores, 188 us now.
 // Every wait is bounded by the global timer; on expiry the CTA records an
 // error in a device word (read by naja_mlp_check), stops issuing, drains its
 // own copies and MMAs and frees its tensor memory.
@@ -44,6 +44,7 @@ namespace {
 
 constexpr int kTileM = 128;
 constexpr int kMaxStages = 16;
+constexpr int kStageSlices = 2;  // K slices per stage: one barrier round trip for both
 constexpr int kThreads = 192;
 constexpr uint64_t kTimeoutNs = 5ull * 1000 * 1000 * 1000;
 constexpr int kStagePad = 32 * 33;  // floats of an epilogue warp's block
@@ -74,7 +75,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const uint32_t stage_bytes = static_cast<uint32_t>(a.a_bytes) + kBTile;
+  const uint32_t slice_bytes = static_cast<uint32_t>(a.a_bytes) + kBTile;
+  const uint32_t stage_bytes = kStageSlices * slice_bytes;
   const int S = a.stages;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(S) * stage_bytes);
   uint64_t* empty = full + kMaxStages;
@@ -113,16 +115,19 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t round = 0, last_parity = 0, used = 0;
       for (long long tile = blockIdx.x; tile < a.tiles && !*abort_flag; tile += gridDim.x) {
         const int tm = static_cast<int>(tile / a.tiles_n), tn = static_cast<int>(tile % a.tiles_n);
-        for (int ks = 0; ks < K; ++ks) {
+        for (int ks = 0; ks < K; ks += kStageSlices) {
           if (round >= 1 && !mbar_wait_bounded(&empty[stage], (round - 1) & 1u, kTimeoutNs)) {
             set_error(err, kGemmTimeoutSlot, static_cast<int>(blockIdx.x), stage, ks);
             *abort_flag = 1;
             break;
           }
           unsigned char* st = smem + static_cast<size_t>(stage) * stage_bytes;
-          mbar_arrive_expect_tx(&full[stage], stage_bytes);
-          tc::tma_load_2d(st, &mA, ks * 64, tm * kTileM, &full[stage]);
-          tc::tma_load_2d(st + a.a_bytes, &mB, ks * 64, tn * TN, &full[stage]);
+          const int ns = min(kStageSlices, K - ks);
+          mbar_arrive_expect_tx(&full[stage], ns * slice_bytes);
+          for (int q = 0; q < ns; ++q) {
+            tc::tma_load_2d(st + q * slice_bytes, &mA, (ks + q) * 64, tm * kTileM, &full[stage]);
+            tc::tma_load_2d(st + q * slice_bytes + a.a_bytes, &mB, (ks + q) * 64, tn * TN, &full[stage]);
+          }
           used |= 1u << stage;
           last_parity = (last_parity & ~(1u << stage)) | ((round & 1u) << stage);
           if (++stage == S) {
@@ -150,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tc::fence_after();
         bool ok = true;
-        for (int ks = 0; ks < K; ++ks) {
+        for (int ks = 0; ks < K; ks += kStageSlices) {
           if (!mbar_wait_bounded(&full[stage], parity, kTimeoutNs)) {
             set_error(err, kGemmTimeoutLoad, static_cast<int>(blockIdx.x), stage, ks);
             *abort_flag = 1;
@@ -161,10 +166,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           const unsigned char* st = smem + static_cast<size_t>(stage) * stage_bytes;
           // (with 64 rows of A, accumulator rows 64-127 come from whatever
           // follows them in shared memory and are not read)
+          for (int q = 0; q < kStageSlices && ks + q < K; ++q, st += slice_bytes) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            tc::mma_bf16(tmem + buf * TN, tc::desc_sw128(st + kk * 32), tc::desc_sw128(st + a.a_bytes + kk * 32), idesc,
-                         (ks > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < 4; ++kk) {
+              tc::mma_bf16(tmem + buf * TN, tc::desc_sw128(st + kk * 32), tc::desc_sw128(st + a.a_bytes + kk * 32), idesc,
+                           (ks + q > 0 || kk > 0) ? 1u : 0u);
+            }
           }
           issued = true;
           tc::commit(&empty[stage]);
@@ -282,7 +289,7 @@ int gemm_tile_n(int M, int N, int sms) {
 
 template <int TN>
 cudaError_t gemm_launch(const CUtensorMap& mA, const CUtensorMap& mB, GemmArgs a, int sms, cudaStream_t stream) {
-  const size_t stage = static_cast<size_t>(a.a_bytes) + TN * 128;
+  const size_t stage = kStageSlices * (static_cast<size_t>(a.a_bytes) + TN * 128);
   a.stages = static_cast<int>(std::min<size_t>(kMaxStages, kRingBudget / stage));
   a.tiles_n = (a.N + TN - 1) / TN;
   a.tiles = static_cast<long long>((a.M + kTileM - 1) / kTileM) * a.tiles_n;
