@@ -73,7 +73,8 @@ DeviceGuard::~DeviceGuard() {
 namespace {
 
 __global__ void pad_convert_kernel(const double* __restrict__ src, long long lds, double* __restrict__ A64,
-                                   float* __restrict__ A32, int m, int d, int lda, int* wide) {
+                                   float* __restrict__ A32, const double* __restrict__ b, int m, int d, int lda,
+                                   int* wide) {
   const long long n = static_cast<long long>(lda) * d;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -82,13 +83,8 @@ __global__ void pad_convert_kernel(const double* __restrict__ src, long long lds
     const double v = (r < m) ? src[c * lds + r] : 0.0;
     A64[i] = v;
     A32[i] = __double2float_rn(v);
-    if (!(fabs(v) <= kScreenMaxA)) *wide = 1;
+    if (!(fabs(v) <= kScreenMaxA) || (c == 0 && r < m && !(fabs(b[r]) <= kScreenMaxB))) *wide = 1;
   }
-}
-
-__global__ void check_rhs_kernel(const double* b, int m, int* wide) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < m && !(fabs(b[r]) <= kScreenMaxB)) *wide = 1;
 }
 
 constexpr unsigned long long kWaitTimeoutNs = 5ull * 1000ull * 1000ull * 1000ull;
@@ -159,6 +155,7 @@ struct SparseStore {
   bool built = false;
   long long nnz = 0;        // nonzeros of the FP64 A
   long long tot32 = 0, tot64 = 0;  // column entries stored, padding included
+  void* arena = nullptr;    // one allocation for the arrays below
   void* cols32 = nullptr;   // (float, int) entries of A32 by columns
   int* cs32 = nullptr;
   int max32 = 0;
@@ -202,13 +199,8 @@ int polytope_device(const naja_polytope* P) { return P ? P->device : 0; }
 namespace sparse_build {
 
 void free_sparse(SparseStore& s) {
-  cudaFree(s.cols32);
-  cudaFree(s.cs32);
-  cudaFree(s.cols64);
-  cudaFree(s.cs64);
+  cudaFree(s.arena);
   for (auto& l : s.lanes) cudaFree(l.ptr);
-  cudaFree(s.row_start);
-  cudaFree(s.row_ent);
   s = SparseStore();
 }
 
@@ -375,12 +367,25 @@ int build_sparse(naja_polytope* P) {
     if (nrow > (1LL << 30)) return fail(NAJA_ERR_UNSUPPORTED, "building compressed rows: too many nonzeros");
   }
   rs[m] = static_cast<int>(nrow);
-  e = cudaMalloc(&S.cols32, static_cast<size_t>(t32) * sizeof(SpE32));
-  if (e == cudaSuccess) e = cudaMalloc(&S.cols64, static_cast<size_t>(t64) * sizeof(SpE64));
-  if (e == cudaSuccess) e = cudaMalloc(&S.cs32, (d + 1) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&S.cs64, (d + 1) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&S.row_start, (m + 1) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&S.row_ent, std::max<long long>(nrow, 1) * sizeof(SpE64));
+  size_t bytes = 0;
+  auto take = [&](size_t n) {
+    const size_t at = bytes;
+    bytes = (bytes + n + 255) / 256 * 256;
+    return at;
+  };
+  const size_t at_c32 = take(static_cast<size_t>(t32) * sizeof(SpE32)), at_c64 = take(static_cast<size_t>(t64) * sizeof(SpE64)),
+               at_s32 = take((d + 1) * sizeof(int)), at_s64 = take((d + 1) * sizeof(int)), at_rs = take((m + 1) * sizeof(int)),
+               at_re = take(std::max<long long>(nrow, 1) * sizeof(SpE64));
+  e = cudaMalloc(&S.arena, bytes);
+  if (e == cudaSuccess) {
+    char* base = static_cast<char*>(S.arena);
+    S.cols32 = base + at_c32;
+    S.cols64 = base + at_c64;
+    S.cs32 = reinterpret_cast<int*>(base + at_s32);
+    S.cs64 = reinterpret_cast<int*>(base + at_s64);
+    S.row_start = reinterpret_cast<int*>(base + at_rs);
+    S.row_ent = base + at_re;
+  }
   if (e == cudaSuccess) e = cudaMemcpy(S.cs32, cs32.data(), (d + 1) * sizeof(int), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(S.cs64, cs64.data(), (d + 1) * sizeof(int), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(S.row_start, rs.data(), (m + 1) * sizeof(int), cudaMemcpyHostToDevice);
@@ -599,24 +604,22 @@ int naja_polytope_create(int device, int m, int d, const double* A, int lda, con
       e = cudaMemcpy(staged, A, static_cast<size_t>(lda) * d * sizeof(double), cudaMemcpyHostToDevice);
     src = staged;
   }
-  if (e == cudaSuccess) e = cudaMemset(P->err, 0, 4 * sizeof(int));
-  if (e == cudaSuccess) {
-    const long long total = static_cast<long long>(P->lda) * d;
-    const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 16));
-    pad_convert_kernel<<<blocks, 256>>>(src, lda, P->A64, P->A32, m, d, P->lda, P->err);
-    e = cudaGetLastError();
-  }
+  if (e == cudaSuccess) e = cudaMemset(P->err, 0, kErrWords * sizeof(int));
   if (e == cudaSuccess)
     e = cudaMemcpy(P->b, b, m * sizeof(double), is_device_ptr(b) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    check_rhs_kernel<<<(m + 255) / 256, 256>>>(P->b, m, P->err);
+    const long long total = static_cast<long long>(P->lda) * d;
+    const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 16));
+    pad_convert_kernel<<<blocks, 256>>>(src, lda, P->A64, P->A32, P->b, m, d, P->lda, P->err);
     e = cudaGetLastError();
   }
-  int wide = 0;
+  int wide = 0;  // (the read below waits for everything above)
   if (e == cudaSuccess) e = cudaMemcpy(&wide, P->err, sizeof(int), cudaMemcpyDeviceToHost);
   P->screen_ok = wide == 0;
-  if (e == cudaSuccess) e = cudaMemset(P->err, 0, 4 * sizeof(int));
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e == cudaSuccess && wide) {
+    e = cudaMemset(P->err, 0, kErrWords * sizeof(int));
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
   if (staged) cudaFree(staged);
   if (e != cudaSuccess) {
     naja_polytope_destroy(P);
