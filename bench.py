@@ -214,6 +214,17 @@ def _chr_launches(W, a, choice):
     return 1
 
 
+def _backmap_launches(W, mode):
+    """Kernels one backmap launches (the chunks of backmap_tc_chunk_rows)."""
+    if mode == "fp64":
+        return 1
+    rows, tiles_n, pairs = W.nspc * W.nchains, -(-W.n // 256), 74
+    most = max(1, (112 << 20) // (2 * (-(-W.d // 64) * 64) * (4 if mode == "tf32x3" else 2) * 256))
+    use = {b: b * tiles_n / (-(-b * tiles_n // pairs) * pairs) for b in range(most, (most + 1) // 2 - 1, -1)}
+    chunk = rows if rows <= most * 256 else 256 * max(use, key=lambda b: (round(use[b], 9), b))
+    return 1 + 2 * -(-rows // chunk)
+
+
 def _headline_traffic(a, W, choice):
     """The captured DRAM bytes of the headline launch, where this run is that
     launch's workload (else None: traffic was not captured for it)."""
@@ -481,7 +492,7 @@ def _ours(a, rank, world):
         "config": W.config(a),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": _headline_traffic(a, W, choice), "peak_source": peak_kind,
-                     "kernel": "chr_sparse_kernel" if choice["kernel"] == "columns" else "chr_kernel",
+                     "kernel": "chr_columns_kernel" if choice["kernel"] == "columns" else "chr_screen_kernel",
                      "kernel_threads": choice["threads"], "kernel_ms": chr_mean,
                      "bytes_per_chr_step": W.bytes_per_step,
                      "bytes_definition": "4 m (1 + p_pair) + 4 d / thinning: one FP32 column per coordinate step, "
@@ -497,17 +508,17 @@ def _ours(a, rank, world):
         "gate": gate,
         "backmap": {"mode": a.backmap_mode, "ms": statistics.mean(bm_ms), "error_vs_fp64": bm_err,
                     "roofline": _backmap_roofline(W, statistics.mean(bm_ms), a.backmap_mode),
-                    # y = M z + c of the rounded job (FP64 SIMT, for the metric), timed apart
+                    # y = M z + c of the rounded job (FP64, for the metric), timed apart
                     "y_map_ms": statistics.mean(ymap_ms),
                     # the reference's backmap_into (src/gpu/backmap.cu:20-48): cuBLAS DGEMM + shift
                     "cublas_dgemm_ms": dgemm_ms},
         "reference_semantics_validate": {k: ref_sem[k] for k in ("status", "ess", "rhat")},
         # per step: the CHR run (one step kernel, or per recompute interval one
         # slack-recompute kernel and one step kernel), the y map (one FP64
-        # kernel) when rounded, then the backmap (one FP64 kernel, or operand
-        # split x2 + tcgen05 GEMM)
+        # kernel) when rounded, then the backmap (one FP64 kernel, or the split
+        # of T and per chunk of samples their split and the tcgen05 GEMM)
         "gpu_launches": a.steps * (_chr_launches(W, a, choice) + (1 if rounded else 0)
-                                   + (1 if a.backmap_mode == "fp64" else 3)),
+                                   + _backmap_launches(W, a.backmap_mode)),
     }
     line["clocks"] = clk.summary()
     detail = {"job_ms": job_ms, "chr_ms": chr_ms, "backmap_ms": bm_ms, "y_map_ms": ymap_ms}
@@ -620,7 +631,7 @@ def _plain_figure(a, W, torch, dev):
     return {"value": min_ess / (statistics.mean(job_ms) / 1e3), "unit": UNIT, "min_ess": min_ess,
             "rhat_max": float(rhat.max()), "ms_per_job": statistics.mean(job_ms), "chr_ms": cm,
             "chr_steps_per_s": W.steps / (cm / 1e3),
-            "roofline": {"kernel": "chr_sparse_kernel" if choice["kernel"] == "columns" else "chr_kernel",
+            "roofline": {"kernel": "chr_columns_kernel" if choice["kernel"] == "columns" else "chr_screen_kernel",
                          "threads": choice["threads"], "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "peak_source": peak_kind,
                          "compressed_bytes_per_chr_step": W.compressed_bytes_per_step}}

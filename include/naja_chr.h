@@ -50,7 +50,7 @@ extern "C" {
 #define NAJA_SPARSE_DENSE 1   /* every row of A every step                                     */
 #define NAJA_SPARSE_COLUMNS 2 /* only the nonzero rows of the step's column(s)                 */
 
-#define NAJA_BACKMAP_FP64 0    /* FP64 SIMT GEMM (reference arithmetic)          */
+#define NAJA_BACKMAP_FP64 0    /* FP64 GEMM (reference arithmetic)               */
 #define NAJA_BACKMAP_BF16X3 1  /* split-BF16 on tcgen05, FP32 accumulate          */
 #define NAJA_BACKMAP_TF32X3 2  /* 3xTF32 on tcgen05, FP32 accumulate              */
 
@@ -149,15 +149,18 @@ int naja_chr_kernel_choice(const naja_polytope* P, const naja_chr_params* params
  * naja_b200/autotune.py, or by hand). */
 typedef struct naja_batch_config {
     int threads;      /* consumer threads per chain: 128, 256 or 512            */
-    int slots;        /* staged-column ring depth 2..8, 0 = direct column reads */
-    int slack_smem;   /* 1: slack in shared memory (several chains per SM)      */
+    int slots;        /* staged-column ring depth 2..8, 0 = direct column reads; the compressed
+                         kernel may take fewer (>= 3) where one more chain per SM fits then */
+    int slack_smem;   /* 1: slack in shared memory, 0: in registers; the screened kernel
+                         (Philox coordinate and pair steps) keeps it in registers */
     int ctas_per_sm;  /* resident chains per SM, 0 = as many as fit             */
     int sparse;       /* 1: compressed-column kernel (threads 64, 128 or 256 consumer
                          threads, slots 3..8, slack_smem ignored); same samples       */
 } naja_batch_config;
 
 /* Runs params->nchains chains of each of `nmodels` polytopes (the same d)
- * in ONE persistent launch.  Model k uses seed params->seed + k*seed_stride
+ * in one persistent launch (per recompute interval one slack kernel and one
+ * launch, where the polytopes have at least 2^19 cells).  Model k uses seed params->seed + k*seed_stride
  * and its chains are numbered 0..nchains-1, so it draws exactly the streams a
  * standalone naja_chr_run of that model with that seed draws.  X0s[k]
  * (d x nchains, leading dimension ldx) and samples[k] ((nspc*nchains) x d,
