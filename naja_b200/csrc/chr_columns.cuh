@@ -161,9 +161,9 @@ __device__ __noinline__ void run_col_producer(const ChrArgs& a, const SpArgs& sp
   const ColShared sh(smem, L);
   const unsigned char* cols = static_cast<const unsigned char*>(sp.lanes);
   const uint32_t col_bytes = static_cast<uint32_t>(L.slot_bytes);
-  const int S = L.slots, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const long long total = launch_steps(a);
-  uint32_t used = 0;
+  RingClaims ring(RES ? 1 : L.slots);  // (resident columns: not used)
   unsigned long long w_empty = 0;
   const unsigned long long p_start = clock64();
   bool stop = false;
@@ -227,26 +227,28 @@ __device__ __noinline__ void run_col_producer(const ChrArgs& a, const SpArgs& sp
     if (lane == 0) mbar_arrive(sh.drawn() + (batch_id & 1));
     if constexpr (!RES) {
       const uint32_t pairs = __ballot_sync(0xffffffffu, kind == kPair);
-      const uint32_t claim = used + lane + __popc(pairs & ((1u << lane) - 1u));
+      // this lane's first claim, counted from the batch's first
+      const uint32_t claim = lane + __popc(pairs & ((1u << lane) - 1u));
+      const int sa = ring.slot(claim), sb = ring.slot(claim + 1);
+      const uint32_t pa = ring.parity(claim), pb = ring.parity(claim + 1);
+      uint32_t claimed = 0;
       for (int k = 0; k < n; ++k) {
         bool ok = true;
         if (lane == k) {
-          const int sa = static_cast<int>(claim % S), sb = static_cast<int>((claim + 1) % S);
-          const uint32_t ra = claim / S, rb = (claim + 1) / S;
           if (bad) {
             set_error(a.err, kDevBadPair, ei, ej, static_cast<int>(t0 + k));
             ok = false;
           }
           const unsigned long long w0 = a.wait_cycles ? clock64() : 0ull;
-          if (ok && ra >= 1 && !wait_free(&sh.empty()[sa], (ra - 1) & 1u, a.timeout_ns, sh.abort_flag())) {
+          if (ok && ring.refill(claim) && !wait_free(&sh.empty()[sa], pa ^ 1u, a.timeout_ns, sh.abort_flag())) {
             if (!*sh.abort_flag())
-              set_error(a.err, kDevTimeoutEmpty, sa, static_cast<int>(ra), static_cast<int>(t0 + k));
+              set_error(a.err, kDevTimeoutEmpty, sa, static_cast<int>(pa), static_cast<int>(t0 + k));
             ok = false;
           }
-          if (ok && kind == kPair && rb >= 1 &&
-              !wait_free(&sh.empty()[sb], (rb - 1) & 1u, a.timeout_ns, sh.abort_flag())) {
+          if (ok && kind == kPair && ring.refill(claim + 1) &&
+              !wait_free(&sh.empty()[sb], pb ^ 1u, a.timeout_ns, sh.abort_flag())) {
             if (!*sh.abort_flag())
-              set_error(a.err, kDevTimeoutEmpty, sb, static_cast<int>(rb), static_cast<int>(t0 + k));
+              set_error(a.err, kDevTimeoutEmpty, sb, static_cast<int>(pb), static_cast<int>(t0 + k));
             ok = false;
           }
           if (a.wait_cycles) w_empty += clock64() - w0;
@@ -265,8 +267,9 @@ __device__ __noinline__ void run_col_producer(const ChrArgs& a, const SpArgs& sp
           stop = true;
           break;
         }
-        used += 1u + ((pairs >> k) & 1u);
+        claimed += 1u + ((pairs >> k) & 1u);
       }
+      ring.advance(claimed);
     }
   }
   if (a.wait_cycles) {
@@ -277,11 +280,11 @@ __device__ __noinline__ void run_col_producer(const ChrArgs& a, const SpArgs& sp
     }
   }
   if constexpr (!RES) {
-    // drain: slot q's last claim is the largest p < used with p % S == q
-    if (lane < S && static_cast<uint32_t>(lane) < used) {
-      const uint32_t last = (used - 1 - lane) / S;
-      if (!mbar_wait_bounded(&sh.full()[lane], last & 1u, a.timeout_ns))
-        set_error(a.err, kDevTimeoutDrain, lane, static_cast<int>(last & 1u), static_cast<int>(used));
+    // drain: no bulk copy may outlive the CTA
+    if (lane < L.slots && ring.used(lane)) {
+      const uint32_t last = ring.last_parity(lane);
+      if (!mbar_wait_bounded(&sh.full()[lane], last, a.timeout_ns))
+        set_error(a.err, kDevTimeoutDrain, lane, static_cast<int>(last), static_cast<int>(ring.next));
     }
     __syncwarp();
   }
