@@ -23,6 +23,7 @@ master weights.  PyTorch only provides device memory and the stream.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -73,8 +74,45 @@ class _Buffers:
     loss: object = None
 
 
+def _record(out, stream):
+    """Tensors of `out` are in use on `stream` too."""
+    if isinstance(out, (list, tuple)):
+        for v in out:
+            _record(v, stream)
+    elif hasattr(out, "record_stream"):
+        out.record_stream(stream)
+
+
+def _on_net_stream(method):
+    """Runs a method's torch calls on the stream that the net's kernels are
+    launched on.  Under another current stream (torch's side streams do not
+    wait for the default one) the net's stream first waits for the caller's,
+    whose work may have made the arguments, and the caller's for the net's
+    after it."""
+
+    @functools.wraps(method)
+    def run(self, *args, **kw):
+        cuda = self.torch.cuda
+        caller, own = cuda.current_stream(self.device), cuda.default_stream(self.device)
+        if caller == own:
+            return method(self, *args, **kw)
+        own.wait_stream(caller)
+        with cuda.stream(own):
+            try:
+                out = method(self, *args, **kw)
+            finally:
+                caller.wait_stream(own)
+        _record(out, caller)
+        return out
+
+    return run
+
+
 class RoundingNet:
-    """dims = (n_in, hidden..., n_out); GELU between layers, linear output."""
+    """dims = (n_in, hidden..., n_out); GELU between layers, linear output.
+
+    All device work is queued on the device's default stream, whatever stream
+    is current at a call; the current stream waits for it."""
 
     def __init__(self, dims, *, seed=0, device="cuda", lr=1e-3, betas=(0.9, 0.999), eps=1e-8):
         import torch
@@ -82,7 +120,7 @@ class RoundingNet:
         self.torch = torch
         self.dims = tuple(int(v) for v in dims)
         self.device = torch.device(device)
-        self.stream = 0
+        self.stream = 0  # the default stream (_on_net_stream)
         self.lr, self.betas, self.eps = lr, betas, eps
         self.step_count = 0
         self.lib = load()
@@ -96,6 +134,7 @@ class RoundingNet:
         self._bufs = {}
 
     # ------------------------------------------------------------ memory
+    @_on_net_stream
     def _make_layer(self, a, b, w, bias):
         t = self.torch
         dev = self.device
@@ -162,8 +201,9 @@ class RoundingNet:
     def _load_targets(self, z, T, n_out):
         """Targets on the host go through a page-locked buffer of the batch
         size's own (several cores fill it, one asynchronous copy empties it,
-        both while the forward pass runs); every call that uses it ends with
-        the stream synchronised."""
+        both while the forward pass runs); the copy and every kernel are on
+        the net's stream, which a call that uses the buffer ends by
+        synchronising."""
         t = self.torch
         T = t.as_tensor(T, dtype=t.float32)
         if not T.is_cuda and z.target_host is None:
@@ -172,6 +212,7 @@ class RoundingNet:
             T = z.target_host.copy_(T)
         z.target[:, :n_out].copy_(T, non_blocking=True)
 
+    @_on_net_stream
     def predict(self, X):
         """X (B, n_in) -> outputs (B, n_out) as a float32 CUDA tensor."""
         X = np.asarray(X, np.float32) if not hasattr(X, "data_ptr") else X
@@ -181,6 +222,7 @@ class RoundingNet:
         check(self.lib.naja_mlp_check(self.stream))
         return z.out[:, : self.dims[-1]].clone()
 
+    @_on_net_stream
     def gradients(self, X, T, w=None):
         """Forward + backward; returns loss and leaves gradients in the layers (no update)."""
         t = self.torch
@@ -216,6 +258,7 @@ class RoundingNet:
         check(self.lib.naja_mlp_check(self.stream))
         return float(z.loss.item())
 
+    @_on_net_stream
     def apply_gradients(self):
         self.step_count += 1
         b1, b2 = self.betas
@@ -232,10 +275,12 @@ class RoundingNet:
         return loss
 
     # ------------------------------------------------------------ state
+    @_on_net_stream
     def snapshot(self):
         """Copies of the FP32 master weights and biases (device tensors)."""
         return [(L.W.clone(), L.b.clone()) for L in self.layers]
 
+    @_on_net_stream
     def restore(self, snap):
         """Loads a snapshot and refreshes the BF16 copies the kernels read."""
         for L, (W, b) in zip(self.layers, snap):
@@ -244,10 +289,12 @@ class RoundingNet:
             check(self.lib.naja_cast_bf16(L.n_out, L.n_in, _p(L.W), L.W.shape[1], _p(L.W_bf), L.W_bf.shape[1],
                                           _p(L.W_bf_t), L.W_bf_t.shape[1], self.stream))
 
+    @_on_net_stream
     def weights(self):
         """[(W (n_out, n_in) float32, b (n_out,))] as numpy arrays."""
         return [(L.W[:, : L.n_in].cpu().numpy(), L.b.cpu().numpy()) for L in self.layers]
 
+    @_on_net_stream
     def weight_grads(self):
         return [(L.gW[:, : L.n_in].cpu().numpy(), L.gb.cpu().numpy()) for L in self.layers]
 
