@@ -191,9 +191,7 @@ int plan_single(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   const int elt = precision == NAJA_PREC_FP64 ? 8 : 4;
   int threads = 0;
   if (tpb > 0) {
-    // The reference's thread counts (chr.cu:529-551).  A block also holds the
-    // producer warp, so 1024 maps to 992 consumer threads.
-    if (tpb != 32 && tpb != 64 && tpb != 128 && tpb != 256 && tpb != 512 && tpb != 1024) return NAJA_ERR_INVALID_ARGUMENT;
+    // a block also holds the producer warp, so 1024 maps to 992 consumer threads
     threads = tpb == 1024 ? 992 : tpb;
   } else {
     // Automatic: at most 12 rows per thread, 992 threads only when 512 would
@@ -336,6 +334,10 @@ int chr_plan(int precision, int m, int d, int lda, int tpb, int max_slots, int n
   (void)nchains;
   (void)sms;
   if (cluster >= 2) return plan_cluster(precision, m, d, tpb, max_slots, cluster, out);
+  // A forced count is one of the reference's (chr.cu:529-551), whatever counts
+  // a kernel has beside them.
+  if (tpb > 0 && tpb != 32 && tpb != 64 && tpb != 128 && tpb != 256 && tpb != 512 && tpb != 1024)
+    return NAJA_ERR_INVALID_ARGUMENT;
   if (screen && plan_screen(precision, m, d, lda, tpb, max_slots, out) == NAJA_OK) return NAJA_OK;
   return plan_single(precision, m, d, lda, tpb, max_slots, out);
 }
