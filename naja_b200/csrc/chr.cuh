@@ -69,8 +69,10 @@ struct ChrLaunchConfig {
   int entries;    // chr_columns.cuh: entries of a column per lane (template capacity)
   int resident;   // chr_columns.cuh: 1 = all columns stay in shared memory (the ring is not used)
   int pair_scatter;  // sparse-column kernel: 1 = pair steps through a scratch column, 0 = by search
+  int uniform;       // chr_kernel: 1 = every warp runs `rows` chunks, the rows past m repeating the last V
+                     // rows (needs m % V == 0); 0 = chunks as rows allow, `rows` the template capacity
   int screen;        // dense single-CTA kernel: 1 = the screened kernel (chr_screen.cuh), `rows` chunks
-                     // per warp exactly; 0 = chr_kernel, `rows` its template capacity
+                     // per warp exactly; 0 = chr_kernel
 };
 
 // Compressed columns of A for the sparse-column kernel, in the tier's

@@ -10,12 +10,14 @@ int chr_launch_float_32(const ChrArgs& a, int nchains, const ChrLaunchConfig& cf
 int chr_launch_float_64(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_128(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_256(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
+int chr_launch_float_448(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_512(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_float_992(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_32(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_64(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_128(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_256(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
+int chr_launch_double_448(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_512(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 int chr_launch_double_992(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream);
 
@@ -184,6 +186,8 @@ __global__ void batch_copy_x_kernel(const ModelDesc* __restrict__ from, const Mo
 // Largest chunks-per-warp capacity used for a thread count (the slack of R
 // chunks takes R * V registers per thread, V rows per lane and chunk).
 int max_chunks_for(int threads, int v) { return (threads <= 512 ? 32 : 16) / v; }
+// Largest chunk count of the uniform-chunk kernels (instantiated 1..8).
+constexpr int kMaxUniformChunks = 8;
 }  // namespace
 
 namespace {
@@ -231,6 +235,27 @@ int plan_single(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   out->entries = 0;
   out->resident = 0;
   out->screen = 0;
+  out->uniform = 0;
+  // Uniform chunks: every warp runs the same R = ceil(chunks / warps) chunks
+  // as one straight-line row pass (rows past m repeat the last V).  Against
+  // chunks tested one by one, us per step, 16 chains: m = 5200 with one
+  // infinite bound 1.64 / 1.94 (FP64 3.33 / 3.66), with k-sparse steps 2.69 /
+  // 3.12 (5.75 / 6.46); m = 1200 with k-sparse steps 1.98 / 2.33 (3.45 / 4.09).
+  const int v = standalone_v(precision), exact = (chunks + warps - 1) / warps;
+  if (m % v == 0 && m >= v && exact <= kMaxUniformChunks && exact <= max_chunks_for(threads, v)) {
+    out->uniform = 1;
+    out->rows = exact;
+    // 14 warps where they hold the same chunks per warp as 16: fewer row
+    // slots repeat (m 5200: 42 for 41 chunks instead of 48); the layout
+    // depends on the thread count, so it is planned again
+    if (tpb <= 0 && threads == 512 && 14 * exact >= chunks) {
+      const Layout L448 = make_layout(d, lda, elt, 448, slots);
+      if (L448.total <= kSmemBudget) {
+        out->threads = 448;
+        out->smem = L448.total;
+      }
+    }
+  }
   return NAJA_OK;
 }
 
@@ -275,6 +300,7 @@ int plan_screen(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
   out->entries = 0;
   out->resident = 0;
   out->screen = 1;
+  out->uniform = 0;
   return NAJA_OK;
 }
 
@@ -320,6 +346,7 @@ int plan_cluster(int precision, int m, int d, int tpb, int max_slots, int cs, Ch
   out->entries = 0;
   out->resident = 0;
   out->screen = 0;
+  out->uniform = 0;
   return NAJA_OK;
 }
 }  // namespace
@@ -361,6 +388,7 @@ int chr_launch(int precision, const ChrArgs& args, int nchains, const ChrLaunchC
     case 64: return f64 ? chr_launch_double_64(args, nchains, cfg, stream) : chr_launch_float_64(args, nchains, cfg, stream);
     case 128: return f64 ? chr_launch_double_128(args, nchains, cfg, stream) : chr_launch_float_128(args, nchains, cfg, stream);
     case 256: return f64 ? chr_launch_double_256(args, nchains, cfg, stream) : chr_launch_float_256(args, nchains, cfg, stream);
+    case 448: return f64 ? chr_launch_double_448(args, nchains, cfg, stream) : chr_launch_float_448(args, nchains, cfg, stream);
     case 512: return f64 ? chr_launch_double_512(args, nchains, cfg, stream) : chr_launch_float_512(args, nchains, cfg, stream);
     case 992: return f64 ? chr_launch_double_992(args, nchains, cfg, stream) : chr_launch_float_992(args, nchains, cfg, stream);
     default: return NAJA_ERR_UNSUPPORTED;

@@ -44,6 +44,7 @@ int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_s
   out->entries = entries;
   out->pair_scatter = 0;
   out->screen = 0;
+  out->uniform = 0;
   return NAJA_OK;
 }
 
@@ -96,6 +97,7 @@ int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, i
   out->resident = 0;
   out->pair_scatter = scatter ? 1 : 0;
   out->screen = 0;
+  out->uniform = 0;
   return NAJA_OK;
 }
 

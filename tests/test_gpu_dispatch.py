@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+import oracle.oracle as O
 from naja_b200 import Polytope
 from naja_b200._lib import InvalidArgument
 
@@ -23,3 +24,40 @@ def test_forced_thread_counts_are_the_references(cuda, tpb):
         P.kernel_choice(10, 1, 2, tpb=tpb)
     with pytest.raises(InvalidArgument, match="Invalid threads per block"):
         P.run(np.zeros(5), 10, 1, 2, tpb=tpb)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_general_kernel_runs_uniform_chunks(cuda, precision):
+    """Runs that divide every row (k-sparse steps, an infinite bound) on 14
+    warps where those hold the rows in as many chunks as 16."""
+    A, b = _dense(5200, 4)
+    P = Polytope(A, b)
+    kw = dict(precision=precision, sparse="dense")
+    assert P.kernel_choice(10, 1, 2, ksparse_prob=0.2, **kw)["threads"] == 448
+    b = b.copy()
+    b[3] = np.inf
+    assert Polytope(A, b).kernel_choice(10, 1, 2, **kw)["threads"] == 448
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("kw", [dict(ksparse_prob=0.3, ksparse_k=3), dict(infinite=True), dict(infinite=True, tpb=1024)], ids=str)
+@pytest.mark.parametrize("m", [6, 8, 132, 642, 1284, 5200])
+def test_general_kernel_against_the_oracle(cuda, m, kw, precision):
+    """Bit for bit (both tiers give the oracle's samples exactly), row counts
+    that are and are not multiples of a lane's rows."""
+    kw = dict(kw)
+    A, b = _dense(m, 5, seed=m)
+    if kw.pop("infinite", False):
+        b[1] = np.inf
+    run = dict(seed=5, pair_prob=0.4, resync_interval=11, precision=precision)
+    P = Polytope(A, b)
+    dt = np.float64 if precision == "fp64" else np.float32
+    slack, sf = np.empty((3, m), dt), np.empty((3, m), dt)
+    got = P.run(np.zeros(5), 25, 3, 3, out_dtype="f64", sparse="dense", slack_final=slack, **run, **kw)
+    P.check()
+    tpb = kw.pop("tpb", None)
+    assert np.array_equal(got, O.chr_run(A, b, np.zeros(5), 25, 3, 3, **run, **kw), equal_nan=True)
+    # with other threads, columns straight from global memory
+    P.run(np.zeros(5), 25, 3, 3, out_dtype="f64", sparse="dense", slack_final=sf, max_slots=2, tpb=tpb or 256, **run, **kw)
+    P.check()
+    assert np.array_equal(slack, sf, equal_nan=True)
