@@ -2,16 +2,15 @@
 // split-R-hat per dim, following src/validate/mcmc.cpp:17-194 of
 // quothbonney/naja.
 //
-// ESS: one CTA per chain and group of coordinates (whole 32-byte sectors of
-// the sample rows).  Each series is centred in shared memory and its
+// ESS: one CTA per series.  The series is centred in shared memory and its
 // autocovariances are summed directly (FP32 products, FP64 sums) in blocks of
-// 64 lags until Geyer's initial positive sequence stops.  The reference
-// obtains the same acov[k] = (1/n) sum (x_t-m)(x_{t+k}-m) from a float FFT of
-// size 2n; the direct sum needs only the lags the rule reaches (a few blocks
-// for a mixing chain) and has no FFT round-off.
+// lags until Geyer's initial positive sequence stops.  The reference obtains
+// the same acov[k] = (1/n) sum (x_t-m)(x_{t+k}-m) from a float FFT of size 2n;
+// the direct sum needs only the lags the rule reaches (a few blocks for a
+// mixing chain) and has no FFT round-off.
 //
-// R-hat: half-chain sums in FP64 as mcmc.cpp takes them, over sample rows as
-// they lie in memory (a lane per coordinate), then one combination.
+// R-hat: half-chain sums in FP64 as mcmc.cpp takes them, eight coordinates (a
+// sector of the sample rows) per CTA.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -50,196 +49,241 @@ __device__ double block_sum(double v, double* scratch) {
   return t;
 }
 
-// Lags of a block, lags per thread (a sliding window: one new value per
-// sample for kEssLags products) and the slices of a series that the threads of
-// one lag group share out.
-constexpr int kEssBlock = 64;
+// Lags per thread: a sliding window, one new value per sample for kEssLags
+// products.  A block of lags is 4 L of them for L lanes of lags; the threads
+// share out the samples in 256 / L slices.
 constexpr int kEssLags = 4;
-constexpr int kEssLanes = kEssBlock / kEssLags;
-constexpr int kEssSlices = kEssThreads / kEssLanes;
-constexpr int kEssPad = kEssBlock + 4;  // zeros behind a series: a product past its end is 0
+constexpr int kEssMaxBlock = 512;
+constexpr int kEssPad = 2 * kEssLags;  // zeros behind a series: a product past its end is 0
 
-// Floats between the series of a CTA: four values of eight series fall on
-// distinct banks.
-__host__ __device__ inline long ess_pitch(long n) { return (n + kEssPad + 27) / 32 * 32 + 4; }
+// Lags of the block that starts at lag `base`: a mixing chain stops within
+// the first few short ones; a block grows with the lags already taken, so that
+// the products past the stop and the rounds of barriers both stay a small
+// share (700 x 16 series of 2,500 samples, correlation 0.999: 5.5 ms with 64
+// lags throughout, 3.9 ms so; 0.98: 2.3 and 1.5 ms).
+__device__ __forceinline__ int ess_block(long base) {
+  return base <= 256 ? 64 : base <= 512 ? 128 : base <= 1536 ? 256 : kEssMaxBlock;
+}
 
-// What bounds it is the conversion of each FP32 product to FP64 (16 per clock
-// and SM), so the gain is in the products not taken: blocks of 64 lags instead
-// of 512 (16 chains x 2,500 samples x 700 coordinates, correlations 0.3 to
-// 0.99, ESS and R-hat with their copies: 3.56 -> 1.71 ms).
+// One CTA per series.  What bounds it is the conversion of each FP32 product
+// to FP64 (16 per clock and SM), so the gain is in the products not taken:
+// first blocks of 64 lags instead of 512, and a stopping rule that takes a
+// block's pairs side by side.  Eight series per CTA, one after another, read
+// whole sectors of the rows but left SMs idle where there are few series
+// (50 x 2 of 2,500, correlation 0.98: 469 us, 81 one by one), and with many
+// the loads are no bound.
 __global__ void __launch_bounds__(kEssThreads) ess_kernel(const float* __restrict__ s, long N, int dim, int nchains,
-                                                        int layout, int group, double* __restrict__ ess) {
+                                                        int layout, double* __restrict__ ess) {
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ double scratch[32];
-  __shared__ double part_lag[kEssSlices][kEssBlock];
-  __shared__ double acov[kEssBlock];
-  __shared__ int stop_flag;
+  __shared__ __align__(16) double part_lag[kEssThreads * kEssLags];  // [slice][lag]
+  __shared__ double pairs[kEssMaxBlock / 2];
+  __shared__ int first_negative;
   __shared__ double tau_sh;
-  float* all = reinterpret_cast<float*>(sm);
-  const long n = N / nchains, pitch = ess_pitch(n);
-  const int c = blockIdx.x % nchains, dd0 = blockIdx.x / nchains * group;
-  const int ng = dim - dd0 < group ? dim - dd0 : group;
-  for (long e = threadIdx.x; e < n * group; e += kEssThreads) {
-    const long i = e / group;
-    const int g = static_cast<int>(e - i * group);
-    if (g < ng) all[g * pitch + i] = s[series_row(layout, c, i, n, nchains) * dim + dd0 + g];
+  float* y = reinterpret_cast<float*>(sm);
+  const long n = N / nchains, series = blockIdx.x;
+  const int c = blockIdx.x % nchains;
+  {
+    const float* src = s + series_row(layout, c, 0, n, nchains) * dim + blockIdx.x / nchains;
+    const long step = static_cast<long>(layout == 0 ? 1 : nchains) * dim;
+    for (int i = threadIdx.x; i < n + kEssPad; i += kEssThreads) y[i] = i < n ? src[i * step] : 0.0f;
   }
-  for (int e = threadIdx.x; e < group * kEssPad; e += kEssThreads)
-    all[(e / kEssPad) * pitch + n + e % kEssPad] = 0.0f;
   __syncthreads();
-  const int li = threadIdx.x % kEssLanes, slice = threadIdx.x / kEssLanes;
-  for (int g = 0; g < ng; ++g) {
-    float* y = all + g * pitch;
-    const long series = static_cast<long>(dd0 + g) * nchains + c;
-    double part = 0.0;
-    for (long i = threadIdx.x; i < n; i += kEssThreads) part += static_cast<double>(y[i]);
-    const double mean = block_sum(part, scratch) / static_cast<double>(n);
-    part = 0.0;
-    for (long i = threadIdx.x; i < n; i += kEssThreads) {
-      const float v = static_cast<float>(static_cast<double>(y[i]) - mean);
-      y[i] = v;
-      part += static_cast<double>(v) * v;
-    }
-    const double var = block_sum(part, scratch) / static_cast<double>(n);  // acov[0]
-    if (var < 1e-30) {
-      if (threadIdx.x == 0) ess[series] = 1.0;
-      continue;
-    }
-    if (threadIdx.x == 0) {
-      stop_flag = 0;
-      tau_sh = 1.0;
-    }
-    __syncthreads();
-    // pair k uses lags 2k-1, 2k, for k = 1 .. kmax-1
-    const long kmax = n / 2;
-    for (long base = 1; base <= 2 * (kmax - 1); base += kEssBlock) {
-      // this thread: lags lag0 .. lag0 + 3 over its slice of t < n - base
-      // (beyond that every product is 0)
-      const long lag0 = base + li * kEssLags, len = n - base;
-      const long t0 = len * slice / kEssSlices, t1 = len * (slice + 1) / kEssSlices;
-      double acc[kEssLags];
-#pragma unroll
-      for (int j = 0; j < kEssLags; ++j) acc[j] = 0.0;
-      // (a window past the padding only holds lags past n - 1: not summed)
-      if (t0 < t1 && lag0 < n) {
-        const long tend = t1 < n + kEssPad - lag0 - kEssLags ? t1 : n + kEssPad - lag0 - kEssLags;
-        const float* yk = y + lag0;
-        float w[kEssLags];
-#pragma unroll
-        for (int j = 0; j < kEssLags; ++j) w[j] = yk[t0 + j];
-        long t = t0;
-        for (; t + kEssLags <= tend; t += kEssLags) {
-          float next[kEssLags];
-#pragma unroll
-          for (int j = 0; j < kEssLags; ++j) next[j] = yk[t + kEssLags + j];
-#pragma unroll
-          for (int u = 0; u < kEssLags; ++u) {
-            const float v = y[t + u];
-#pragma unroll
-            for (int j = 0; j < kEssLags; ++j)
-              acc[j] += static_cast<double>(v * (u + j < kEssLags ? w[(u + j) % kEssLags] : next[(u + j) % kEssLags]));
-          }
-#pragma unroll
-          for (int j = 0; j < kEssLags; ++j) w[j] = next[j];
-        }
-        for (; t < tend; ++t) {
-          const float v = y[t];
-#pragma unroll
-          for (int j = 0; j < kEssLags; ++j) acc[j] += static_cast<double>(v * yk[t + j]);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kEssLags; ++j) part_lag[slice][li * kEssLags + j] = acc[j];
-      __syncthreads();
-      if (threadIdx.x < kEssBlock) {
-        double a = 0.0;
-#pragma unroll
-        for (int q = 0; q < kEssSlices; ++q) a += part_lag[q][threadIdx.x];
-        acov[threadIdx.x] = a / static_cast<double>(n);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double tau = tau_sh;
-        // acov[i] holds lag base + i; base is odd, so pairs are (i, i+1) for even i.
-        for (int i = 0; i < kEssBlock; i += 2) {
-          const long k = (base + i + 1) / 2;
-          if (k >= kmax) {
-            stop_flag = 1;
-            break;
-          }
-          const double pair = acov[i] / var + acov[i + 1] / var;
-          if (pair < 0.0) {
-            stop_flag = 1;
-            break;
-          }
-          tau += 2.0 * pair;
-        }
-        tau_sh = tau;
-      }
-      __syncthreads();
-      if (stop_flag) break;
-    }
-    if (threadIdx.x == 0) {
-      double tau = tau_sh < 1.0 ? 1.0 : tau_sh;
-      ess[series] = static_cast<double>(n) / tau;
-    }
-    __syncthreads();
+  double part = 0.0;
+  for (long i = threadIdx.x; i < n; i += kEssThreads) part += static_cast<double>(y[i]);
+  const double mean = block_sum(part, scratch) / static_cast<double>(n);
+  part = 0.0;
+  for (long i = threadIdx.x; i < n; i += kEssThreads) {
+    const float v = static_cast<float>(static_cast<double>(y[i]) - mean);
+    y[i] = v;
+    part += static_cast<double>(v) * v;
   }
-}
-
-// Sums and sums of squares of half-chain j (blockIdx.x % 2k) for 32 coordinates,
-// sums[(j * dim + dd) * 2].
-__global__ void __launch_bounds__(256) rhat_sums_kernel(const float* __restrict__ s, long N, int dim, int nchains,
-                                                        int layout, double* __restrict__ sums) {
-  __shared__ double part[2][8][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int j = blockIdx.x % (2 * nchains), dd = blockIdx.x / (2 * nchains) * 32 + lane, c = j / 2, h = j % 2;
-  const long spc = N / nchains, half = spc / 2;
-  double ps = 0.0, ps2 = 0.0;
-  if (dd < dim) {
+  const double var = block_sum(part, scratch) / static_cast<double>(n);  // acov[0]
+  if (var < 1e-30) {
+    if (threadIdx.x == 0) ess[series] = 1.0;
+    return;
+  }
+  if (threadIdx.x == 0) {
+    first_negative = kEssMaxBlock;
+    tau_sh = 1.0;
+  }
+  // pair k uses lags 2k-1, 2k, for k = 1 .. kmax-1
+  const long kmax = n / 2;
+  int block;
+  for (long base = 1; base <= 2 * (kmax - 1); base += block) {
+    block = ess_block(base);
+    const int lanes = block / kEssLags, slices = kEssThreads / lanes;
+    const int li = threadIdx.x & (lanes - 1), slice = threadIdx.x / lanes;
+    // this thread: lags lag0 .. lag0 + 3 over its slice of t < n - lag0
+    // (beyond that every product is 0)
+    const long lag0 = base + li * kEssLags;
+    double acc[kEssLags];
+#pragma unroll
+    for (int j = 0; j < kEssLags; ++j) acc[j] = 0.0;
+    if (lag0 < n) {
+      const int len = static_cast<int>(n - lag0);
+      const int t0 = static_cast<int>(static_cast<long>(len) * slice / slices);
+      const int t1 = static_cast<int>(static_cast<long>(len) * (slice + 1) / slices);
+      const float* yk = y + lag0;
+      float w[kEssLags];
+#pragma unroll
+      for (int j = 0; j < kEssLags; ++j) w[j] = yk[t0 + j];
+      int t = t0;
 #pragma unroll 4
-    for (long i = w; i < half; i += 8) {
-      const double v = static_cast<double>(s[series_row(layout, c, h * half + i, spc, nchains) * dim + dd]);
-      ps += v;
-      ps2 += v * v;
+      for (; t + kEssLags <= t1; t += kEssLags) {
+        float next[kEssLags];
+#pragma unroll
+        for (int j = 0; j < kEssLags; ++j) next[j] = yk[t + kEssLags + j];
+#pragma unroll
+        for (int u = 0; u < kEssLags; ++u) {
+          const float v = y[t + u];
+#pragma unroll
+          for (int j = 0; j < kEssLags; ++j)
+            acc[j] += static_cast<double>(v * (u + j < kEssLags ? w[(u + j) % kEssLags] : next[(u + j) % kEssLags]));
+        }
+#pragma unroll
+        for (int j = 0; j < kEssLags; ++j) w[j] = next[j];
+      }
+      for (; t < t1; ++t) {
+        const float v = y[t];
+#pragma unroll
+        for (int j = 0; j < kEssLags; ++j) acc[j] += static_cast<double>(v * yk[t + j]);
+      }
     }
+#pragma unroll
+    for (int j = 0; j < kEssLags; ++j) part_lag[slice * block + li * kEssLags + j] = acc[j];
+    __syncthreads();
+    // base is odd: thread p has the pair of lags base + 2p, base + 2p + 1
+    if (2 * threadIdx.x < static_cast<unsigned>(block)) {
+      double a = 0.0, b = 0.0;
+      for (int q = 0; q < slices; ++q) {
+        const double2 v = *reinterpret_cast<const double2*>(part_lag + q * block + 2 * threadIdx.x);
+        a += v.x;
+        b += v.y;
+      }
+      const double pair = a / static_cast<double>(n) / var + b / static_cast<double>(n) / var;
+      pairs[threadIdx.x] = pair;
+      if ((base + 1) / 2 + threadIdx.x >= kmax || pair < 0.0) atomicMin(&first_negative, threadIdx.x);
+    }
+    __syncthreads();
+    const int keep = first_negative;
+    if (threadIdx.x == 0) {
+      double tau = tau_sh;
+      const int m = keep < block / 2 ? keep : block / 2;
+#pragma unroll 8
+      for (int p = 0; p < m; ++p) tau += 2.0 * pairs[p];
+      tau_sh = tau;
+    }
+    if (keep < block / 2) break;
   }
-  part[0][w][lane] = ps;
-  part[1][w][lane] = ps2;
-  __syncthreads();
-  if (w < 2 && dd < dim) {
-    double t = 0.0;
-    for (int q = 0; q < 8; ++q) t += part[w][q][lane];
-    sums[(static_cast<size_t>(j) * dim + dd) * 2 + w] = t;
+  if (threadIdx.x == 0) {
+    double tau = tau_sh < 1.0 ? 1.0 : tau_sh;
+    ess[series] = static_cast<double>(n) / tau;
   }
 }
 
-__global__ void rhat_kernel(const double* __restrict__ sums, long N, int dim, int nchains, double* __restrict__ rhat) {
-  const int dd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dd >= dim) return;
-  const long half = N / nchains / 2;
+// Split-R-hat of `group` coordinates per CTA.  A warp's lanes are coordinates
+// by rows; `subs` half-chains at a time have 32 / subs warps each.  Their means
+// stay in shared memory for the spread, or, where there are too many (keep
+// false), are taken a second time: no scratch, whose allocation alone took
+// 100 us after a synchronisation.  What bounds it is loads in flight, so
+// each lane issues kRhatLoads before it adds: 700 x 16 series of 2,500 samples
+// 160 -> 44 us (of 12,500: 419 -> 171), 50 x 4: 119 -> 15 us.
+constexpr int kRhatThreads = 1024;
+constexpr int kRhatWarps = kRhatThreads / 32;
+constexpr int kRhatLoads = 8;
+__global__ void __launch_bounds__(kRhatThreads) rhat_kernel(const float* __restrict__ s, long N, int dim, int nchains,
+                                                            int layout, int lg_group, int subs, bool keep,
+                                                            double* __restrict__ rhat) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ double part[kRhatWarps][8][2];
+  __shared__ double round_mean[kRhatWarps][8], round_var[kRhatWarps][8];
+  double* mean_sh = reinterpret_cast<double*>(sm);  // [half-chain][coordinate]
+  const int group = 1 << lg_group, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane & (group - 1), warps = kRhatWarps / subs, sub = warp / warps;
+  const int row0 = (warp % warps) * (32 >> lg_group) + (lane >> lg_group), rows = warps * (32 >> lg_group);
+  const int dd = blockIdx.x * group + g;
+  const long spc = N / nchains, half = spc / 2;
+  const long step = static_cast<long>(layout == 0 ? 1 : nchains) * dim;
   const int m = 2 * nchains;
-  double grand = 0.0, W = 0.0;
-  // half-chain means and Bessel-corrected variances
-  for (int j = 0; j < m; ++j) {
-    const double* q = sums + (static_cast<size_t>(j) * dim + dd) * 2;
-    const double mean = q[0] / half;
-    double var = (q[1] / half) - mean * mean;
-    var = var * half / (half - 1);
-    grand += mean;
-    W += var;
+  // means and Bessel-corrected variances of half-chains j0 .. j0 + subs - 1
+  auto round = [&](int j0) {
+    double ps = 0.0, ps2 = 0.0;
+    const int j = j0 + sub;
+    if (dd < dim && j < m) {
+      const float* src = s + series_row(layout, j / 2, (j % 2) * half, spc, nchains) * dim + dd;
+      const long at = rows * step;
+      const float* q = src + row0 * step;
+      int i = row0;
+      for (; i + (kRhatLoads - 1) * rows < half; i += kRhatLoads * rows, q += kRhatLoads * at) {
+        float v[kRhatLoads];
+#pragma unroll
+        for (int u = 0; u < kRhatLoads; ++u) v[u] = q[u * at];
+#pragma unroll
+        for (int u = 0; u < kRhatLoads; ++u) {
+          const double x = static_cast<double>(v[u]);
+          ps += x;
+          ps2 += x * x;
+        }
+      }
+      for (; i < half; i += rows, q += at) {
+        const double x = static_cast<double>(*q);
+        ps += x;
+        ps2 += x * x;
+      }
+    }
+    for (int o = 16; o >= group; o >>= 1) {
+      ps += __shfl_xor_sync(0xffffffffu, ps, o);
+      ps2 += __shfl_xor_sync(0xffffffffu, ps2, o);
+    }
+    if (lane < group) {
+      part[warp][lane][0] = ps;
+      part[warp][lane][1] = ps2;
+    }
+    __syncthreads();
+    if (threadIdx.x < subs * group) {
+      const int q = threadIdx.x >> lg_group;
+      double S = 0.0, S2 = 0.0;
+      for (int w = q * warps; w < (q + 1) * warps; ++w) {
+        S += part[w][g][0];
+        S2 += part[w][g][1];
+      }
+      const double mean = S / half;
+      const double var = (S2 / half) - mean * mean;
+      round_mean[q][g] = mean;
+      round_var[q][g] = var * half / (half - 1);
+      if (keep && j0 + q < m) mean_sh[(j0 + q) * group + g] = mean;
+    }
+    __syncthreads();
+  };
+  double grand = 0.0, W = 0.0;  // thread g < group
+  for (int j0 = 0; j0 < m; j0 += subs) {
+    round(j0);
+    if (threadIdx.x < group) {
+      for (int q = 0; q < subs && j0 + q < m; ++q) {
+        grand += round_mean[q][g];
+        W += round_var[q][g];
+      }
+    }
   }
   // B: squared deviations from the grand mean
   const double gm = grand / m;
   double B = 0.0;
-  for (int j = 0; j < m; ++j) {
-    const double mean = sums[(static_cast<size_t>(j) * dim + dd) * 2] / half;
-    B += (mean - gm) * (mean - gm);
+  for (int j0 = 0; j0 < m; j0 += subs) {
+    if (!keep) round(j0);
+    if (threadIdx.x < group) {
+      for (int q = 0; q < subs && j0 + q < m; ++q) {
+        const double mean = keep ? mean_sh[(j0 + q) * group + g] : round_mean[q][g];
+        B += (mean - gm) * (mean - gm);
+      }
+    }
   }
-  B *= static_cast<double>(half) / (m - 1);
-  W /= m;
-  const double var_hat = ((half - 1.0) / half) * W + B / half;
-  rhat[dd] = (W > 1e-30) ? sqrt(var_hat / W) : 1.0;
+  if (threadIdx.x < group && dd < dim) {
+    B *= static_cast<double>(half) / (m - 1);
+    W /= m;
+    const double var_hat = ((half - 1.0) / half) * W + B / half;
+    rhat[dd] = (W > 1e-30) ? sqrt(var_hat / W) : 1.0;
+  }
 }
 
 }  // namespace
@@ -263,7 +307,7 @@ extern "C" int naja_validate(const float* samples, long long N, int dim, int nch
                                           " samples per chain");
   if (int st = require_local("naja_validate", {samples, ess, rhat})) return st;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  DeviceBuffer bs, be, br, bsum;
+  DeviceBuffer bs, be, br;
   const void* ds = nullptr;
   int st = device_view(samples, static_cast<size_t>(N) * dim * sizeof(float), stream, bs, &ds);
   if (st) return st;
@@ -278,22 +322,24 @@ extern "C" int naja_validate(const float* samples, long long N, int dim, int nch
     if ((st = br.alloc(static_cast<size_t>(dim) * sizeof(double), stream))) return st;
     dr = static_cast<double*>(br.ptr);
   }
-  if (rhat && (st = bsum.alloc(static_cast<size_t>(4) * nchains * dim * sizeof(double), stream))) return st;
   if (ess) {
-    // eight coordinates per CTA (whole sectors) where they leave room for
-    // another CTA, fewer for long series
-    int group = 8;
-    while (group > 1 && group * ess_pitch(spc) * sizeof(float) > (group > 4 ? 100u : 200u) * 1024) group /= 2;
-    const size_t smem = group * ess_pitch(spc) * sizeof(float);
+    const size_t smem = (static_cast<size_t>(spc) + kEssPad) * sizeof(float);
     cudaFuncSetAttribute(ess_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    ess_kernel<<<static_cast<unsigned>((dim + group - 1) / group) * nchains, kEssThreads, smem, stream>>>(
-        static_cast<const float*>(ds), static_cast<long>(N), dim, nchains, layout, group, de);
+    ess_kernel<<<dim * nchains, kEssThreads, smem, stream>>>(static_cast<const float*>(ds), static_cast<long>(N), dim,
+                                                             nchains, layout, de);
   }
   if (rhat) {
-    rhat_sums_kernel<<<static_cast<unsigned>((dim + 31) / 32) * 2 * nchains, 256, 0, stream>>>(
-        static_cast<const float*>(ds), static_cast<long>(N), dim, nchains, layout, static_cast<double*>(bsum.ptr));
-    rhat_kernel<<<(dim + 127) / 128, 128, 0, stream>>>(static_cast<const double*>(bsum.ptr), static_cast<long>(N), dim,
-                                                       nchains, dr);
+    // eight coordinates per CTA (whole sectors of the rows), fewer where there
+    // are no more; as many half-chains side by side as there are, up to a warp each
+    int lg = 3, subs = 1;
+    while (lg > 0 && (1 << (lg - 1)) >= dim) --lg;
+    while (subs < kRhatWarps && subs < 2 * nchains) subs *= 2;
+    const size_t means = (static_cast<size_t>(2) * nchains * sizeof(double)) << lg;
+    const bool keep = means <= 128 * 1024;
+    const size_t smem = keep ? means : 0;
+    cudaFuncSetAttribute(rhat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    rhat_kernel<<<static_cast<unsigned>((dim + (1 << lg) - 1) >> lg), kRhatThreads, smem, stream>>>(
+        static_cast<const float*>(ds), static_cast<long>(N), dim, nchains, layout, lg, subs, keep, dr);
   }
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && host_e)
