@@ -61,3 +61,34 @@ def test_general_kernel_against_the_oracle(cuda, m, kw, precision):
     P.run(np.zeros(5), 25, 3, 3, out_dtype="f64", sparse="dense", slack_final=sf, max_slots=2, tpb=tpb or 256, **run, **kw)
     P.check()
     assert np.array_equal(slack, sf, equal_nan=True)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("m,pair", [(120, 0.4), (700, 1.0), (5200, 0.4)])
+def test_rows_of_zero_width(cuda, m, pair, precision):
+    """Steps that divide every row among screened ones, bit for bit: two
+    opposite rows that leave half of the coordinates no room."""
+    A, b = _dense(m, 6, seed=m)
+    row = np.concatenate([np.ones(3), np.zeros(3)])
+    A, b = np.vstack([A, row, -row]), np.concatenate([b, [0.0, 0.0]])
+    run = dict(seed=5, pair_prob=pair, resync_interval=11, precision=precision)
+    P = Polytope(A, b)
+    got = P.run(np.zeros(6), 25, 4, 3, out_dtype="f64", sparse="dense", **run)
+    P.check()
+    assert np.array_equal(got, O.chr_run(A, b, np.zeros(6), 25, 4, 3, **run), equal_nan=True)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_resident_columns_only_where_the_chains_fit(cuda, precision):
+    """The unit cube of d = 400: all columns in shared memory for few chains,
+    a ring of them where the copies would keep chains waiting; same samples."""
+    d = 400
+    P = Polytope(np.vstack([np.eye(d), -np.eye(d)]), np.concatenate([np.ones(d), np.zeros(d)]))
+    kw = dict(seed=5, pair_prob=0.3, precision=precision)
+    few, many = P.kernel_choice(4, 8, 3, **kw), P.kernel_choice(4, 8, 600, **kw)
+    assert few["kernel"] == many["kernel"] == "columns"
+    assert few["smem"] > 100 << 10 and many["smem"] < 40 << 10, (few, many)
+    a = P.run(np.full(d, 0.5), 4, 8, 3, **kw)
+    b = P.run(np.full(d, 0.5), 4, 8, 600, **kw)
+    P.check()
+    assert np.array_equal(a.reshape(4, 3, d), b.reshape(4, 600, d)[:, :3])
