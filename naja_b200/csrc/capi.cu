@@ -525,7 +525,8 @@ int choose_kernel(const naja_polytope* P, const naja_chr_params* p, ChrLaunchCon
         const void* lanes = nullptr;
         if (int e = sparse_build::ensure_lanes(Pm, f64, k, 0, cap == cudaStreamCaptureStatusNone, &lanes)) return e;
         if (lanes)
-          st = chr_columns_plan(p->precision, P->m, P->d, nw, S.lane_entries[f64][k], p->max_slots, cfg);
+          st = chr_columns_plan(p->precision, P->m, P->d, nw, S.lane_entries[f64][k], p->max_slots, p->nchains,
+                                sms, cfg);
         if (st == NAJA_OK) spa->lanes = lanes;
       }
       if (st) st = chr_sparse_plan(p->precision, P->m, P->d, max_col, mean, p->tpb, p->max_slots, cfg);

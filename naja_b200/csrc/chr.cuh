@@ -109,9 +109,11 @@ int chr_sparse_plan(int precision, int m, int d, int max_col, double mean_col, i
 // Row warps of chr_columns.cuh's kernel: tpb / 32 when forced (0 where it has
 // none), else from the mean column length.
 int chr_columns_warps(double mean_col, int tpb);
-// Plans it for `nw` row warps and `entries` per lane (1, 2, 3, 4, 5, 6 or 8).
-// NAJA_ERR_UNSUPPORTED where the chain's state does not fit.
-int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, ChrLaunchConfig* out);
+// Plans it for `nw` row warps and `entries` per lane (1, 2, 3, 4, 5, 6 or 8),
+// `nchains` chains on `sms` SMs.  NAJA_ERR_UNSUPPORTED where the chain's state
+// does not fit.
+int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, int nchains, int sms,
+                     ChrLaunchConfig* out);
 // Launches the kernel cfg plans (columns: chr_columns.cuh, else chr_sparse.cuh).
 int chr_sparse_launch(int precision, const ChrArgs& args, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg,
                       cudaStream_t stream);

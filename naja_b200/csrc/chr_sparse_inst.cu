@@ -24,15 +24,27 @@ int chr_columns_warps(double mean_col, int tpb) {
   return nw;
 }
 
-int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, ChrLaunchConfig* out) {
+int chr_columns_plan(int precision, int m, int d, int nw, int entries, int max_slots, int nchains, int sms,
+                     ChrLaunchConfig* out) {
   const int elt = precision == NAJA_PREC_FP64 ? 8 : 4;
   auto bytes = [&](int slots) { return make_col_layout(d, m, elt, nw, entries, slots).total; };
   int slots = kMaxSlots;
   if (max_slots > 0 && max_slots < slots) slots = max_slots;
   while (slots >= 3 && bytes(slots) > kSmemBudget) --slots;
   if (slots < 3) return NAJA_ERR_UNSUPPORTED;
-  // all columns in shared memory where they fit beside the chain's state
-  out->resident = nw <= 2 && max_slots <= 0 && bytes(0) <= kSmemBudget;
+  // All columns in shared memory where they fit beside the chain's state and
+  // the launch's chains do not take longer for it: the registers let 5 chains
+  // (two row warps: 4) run on an SM, not as many copies of the columns may fit,
+  // and a step with them there takes about 3/4 of one with staged columns.  ms
+  // for 1,000 steps in the unit cube of d = 400, resident / staged: 4 chains
+  // FP32 0.42 / 0.54, FP64 0.59 / 0.64; 600 chains 1.27 / 0.70, 2.87 / 0.83; d
+  // = 200, 2,400 chains FP32 2.14 / 2.48.
+  const int most = nw == 1 ? 5 : 4;
+  auto rounds = [&](int q) {
+    const int fit = static_cast<int>((kSmemBudget + 1024) / (bytes(q) + 1024)), per = fit < most ? fit : most;
+    return (nchains + sms * per - 1) / (sms * per);
+  };
+  out->resident = nw <= 2 && max_slots <= 0 && bytes(0) <= kSmemBudget && 3 * rounds(0) <= 4 * rounds(slots);
   out->threads = nw * 32;
   out->rows = 0;
   out->slots = slots;
