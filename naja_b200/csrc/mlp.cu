@@ -279,12 +279,28 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-// The widest tile that still makes two tiles per SM, else the narrowest.
-int gemm_tile_n(int M, int N, int sms) {
-  const long long rows = (M + kTileM - 1) / kTileM;
-  for (int tn : {128, 64, 32})
-    if (rows * ((N + tn - 1) / tn) >= 2LL * sms) return tn;
-  return 16;
+// The tile width that takes the fewest cycles by this account, the narrowest
+// of equals: a CTA's tiles follow one another, each as long as the longer of
+// its slices' way into shared memory (61 bytes a cycle) and its epilogue (28
+// cycles a column), which overlap, and 380 cycles to start; the shorter of the
+// two stands alone once.  us at 16 / 32 / 64 / 128 columns: 4096 x 512 x 23100
+// 620 / 364 / 192 / 113, 2048 x 512 x 2600 53 / 32 / 24 / 30, 64 x 512 x 23100
+// 98 / 98 / 100 / 102, 512 x 2600 x 64 17.0 / 15.8 / 16.9 / 16.3; the widest
+// tile that makes two per SM, whatever K, took 364 and 53 us for the first two.
+int gemm_tile_n(int M, int N, int K, int a_rows, int sms) {
+  const long long rows = (M + kTileM - 1) / kTileM, slices = (K + 63) / 64;
+  int best = 16;
+  long long least = 0;
+  for (int tn : {16, 32, 64, 128}) {
+    const long long rounds = (rows * ((N + tn - 1) / tn) + sms - 1) / sms;
+    const long long load = slices * (a_rows * 128 + tn * 128) / 61, store = 28 * tn;
+    const long long cycles = rounds * (std::max(load, store) + 380) + std::min(load, store);
+    if (least == 0 || cycles < least) {
+      least = cycles;
+      best = tn;
+    }
+  }
+  return best;
 }
 
 template <int TN>
@@ -450,7 +466,7 @@ int naja_gemm_bf16(int M, int N, int K, const void* A, int lda, const void* B, i
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tn = gemm_tile_n(M, N, sms), a_rows = M <= 64 ? 64 : kTileM;
+  const int a_rows = M <= 64 ? 64 : kTileM, tn = gemm_tile_n(M, N, K, a_rows, sms);
   CUtensorMap mA, mB;
   if (!tc::make_map_bf16(&mA, A, M, K, lda, a_rows) || !tc::make_map_bf16(&mB, B, N, K, ldb, tn))
     return fail(NAJA_ERR_CUDA, "naja_gemm_bf16: cuTensorMapEncodeTiled failed");
