@@ -93,9 +93,10 @@ def _on_net_stream(method):
     @functools.wraps(method)
     def run(self, *args, **kw):
         cuda = self.torch.cuda
-        caller, own = cuda.current_stream(self.device), cuda.default_stream(self.device)
-        if caller == own:
+        caller = cuda.current_stream(self.device)
+        if caller.cuda_stream == self.stream:
             return method(self, *args, **kw)
+        own = cuda.default_stream(self.device)
         own.wait_stream(caller)
         with cuda.stream(own):
             try:
@@ -225,6 +226,9 @@ class RoundingNet:
     @_on_net_stream
     def gradients(self, X, T, w=None):
         """Forward + backward; returns loss and leaves gradients in the layers (no update)."""
+        return self._gradients(X, T, w)
+
+    def _gradients(self, X, T, w):
         t = self.torch
         B = int(X.shape[0])
         z = self._buffers(B)
@@ -260,6 +264,9 @@ class RoundingNet:
 
     @_on_net_stream
     def apply_gradients(self):
+        self._apply_gradients()
+
+    def _apply_gradients(self):
         self.step_count += 1
         b1, b2 = self.betas
         for L in self.layers:
@@ -269,9 +276,10 @@ class RoundingNet:
             check(self.lib.naja_adam(1, L.n_out, _p(L.b), _p(L.gb), _p(L.mb), _p(L.vb), L.n_out, self.lr, b1, b2,
                                      self.eps, self.step_count, None, 0, None, 0, self.stream))
 
+    @_on_net_stream
     def train_step(self, X, T, w=None) -> float:
-        loss = self.gradients(X, T, w)
-        self.apply_gradients()
+        loss = self._gradients(X, T, w)
+        self._apply_gradients()
         return loss
 
     # ------------------------------------------------------------ state
