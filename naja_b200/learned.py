@@ -83,6 +83,12 @@ def _record(out, stream):
         out.record_stream(stream)
 
 
+def _current_handle(torch, device):
+    """The current stream's handle, without the 4 us that a Stream object takes."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
 def _on_net_stream(method):
     """Runs a method's torch calls on the stream that the net's kernels are
     launched on.  Under another current stream (torch's side streams do not
@@ -92,11 +98,10 @@ def _on_net_stream(method):
 
     @functools.wraps(method)
     def run(self, *args, **kw):
-        cuda = self.torch.cuda
-        caller = cuda.current_stream(self.device)
-        if caller.cuda_stream == self.stream:
+        if _current_handle(self.torch, self.device) == self.stream:
             return method(self, *args, **kw)
-        own = cuda.default_stream(self.device)
+        cuda = self.torch.cuda
+        caller, own = cuda.current_stream(self.device), cuda.default_stream(self.device)
         own.wait_stream(caller)
         with cuda.stream(own):
             try:

@@ -30,6 +30,7 @@ def test_copies_and_kernels_share_a_stream(monkeypatch):
         def __getattr__(self, name):
             return lambda *a: log.append((name, a[-1], current[-1].cuda_stream)) or 0
 
+    monkeypatch.setattr(learned, "_current_handle", lambda torch, device: current[-1].cuda_stream)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: current[-1])
     monkeypatch.setattr(torch.cuda, "default_stream", lambda device=None: own)
     monkeypatch.setattr(torch.cuda, "stream", use)
