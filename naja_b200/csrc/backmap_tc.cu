@@ -552,7 +552,8 @@ int enqueue_rows(int n, int d, long long N, const void* Y, int y_dtype, const vo
 
 }  // namespace
 
-// Samples split and mapped at a time: the split operands of a chunk stay in L2
+// Samples that naja_backmap splits and maps at a time (the overlapped pipeline
+// maps a chunk of its chains at one go): the split operands of a chunk stay in L2
 // between the kernel that writes them and the GEMM that reads them (about 112
 // MB beside T's), a call's scratch does not grow with its samples, and the
 // chunk's tiles fill whole rounds of the pairs of SMs as well as any number of

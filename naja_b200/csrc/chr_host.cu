@@ -261,14 +261,22 @@ int plan_single(int precision, int m, int d, int lda, int tpb, int max_slots, Ch
 
 // The screened kernel, where the rows fit its registers and three columns its
 // shared memory.  Automatic thread count: the fewest threads that hold the
-// rows in at most 5 chunks per warp, up to 192 (FP64 256) threads, then 448.
-// A step's chain of latencies grows with the warps that meet at its barrier,
-// its instructions per warp with the chunks; measured on 16 chains, us per
-// step (FP32): m = 500: 0.498 with 32 threads, 0.532 with 128, 0.592 with
-// 448; m = 1200: 0.540 with 64, 0.594 with 128; m = 2500: 0.663 with 128,
-// 0.701 with 448; m = 5200: 0.969 with 448, 1.057 with 256, 1.227 with 512.
-// FP64: m = 1200: 0.967 with 128, 1.015 with 448; m = 2500: 1.043 with 256,
-// 1.104 with 512; m = 5200: 1.420 with 448, 2.191 with 512 (which spills).
+// rows in at most 5 chunks per warp, up to 192 (FP64 256) threads, then 448,
+// then 512.  A step's chain of latencies grows with the warps that meet at its
+// barrier, its instructions per warp with the chunks.  us per step, 16 chains,
+// with 32 / 64 / 128 / 256 / 448 / 512 threads (- where the rows do not fit):
+//   FP32 m =   500: 0.54 / 0.53 / 0.55 / 0.59 /    / 0.64
+//        m = 1,200: - / 0.58 / 0.63 / 0.63 /    / 0.65
+//        m = 2,500: - / - / 0.68 / 0.73 /    / 0.80
+//        m = 5,200: - / - / - / 0.99 / 0.92 / 1.19
+//        m = 8,000: - / - / - / 1.45 / 1.43 / 1.45
+//        m = 14,300: - / - / - / - / 2.56 / 3.37
+//   FP64 m =   500: 1.00 / 0.92 / 0.94 / 0.96 /    / 1.06
+//        m = 2,500: - / - / - / 1.08 /    / 1.12
+//        m = 5,200: - / - / - / - / 1.35 / 2.09
+// More than 5 (512 threads: 2) chunks per warp spill registers; the forms that
+// spill are still the faster ones: chr_kernel takes 1.96 us at m = 8,000 and
+// 4.54 at 14,000, and more warps than 16 cannot hold a next column.
 int plan_screen(int precision, int m, int d, int lda, int tpb, int max_slots, ChrLaunchConfig* out) {
   const bool f64 = precision == NAJA_PREC_FP64;
   const int elt = f64 ? 8 : 4;
@@ -479,8 +487,9 @@ int chr_batch_plan(int m_max, int d, int lda_max, bool quick, BatchConfig* cfg) 
   const int nt = cfg->threads;
   if (nt != 128 && nt != 256 && nt != 512) return NAJA_ERR_INVALID_ARGUMENT;
   const int chunks = (m_max + 32 * kBatchV - 1) / (32 * kBatchV), warps = nt / 32;
-  // The screened kernel where the slots it would run with, and as many chains
-  // per SM as asked for, fit.
+  // The screened kernel where its rows and the slots asked for fit; as many
+  // chains run per SM as its registers and shared memory let, at most those
+  // asked for.
   cfg->screen = 0;
   if (quick && cfg->slots >= 3 && cfg->slots <= kMaxSlots && (chunks + warps - 1) / warps <= screen_batch_max_chunks(nt)) {
     const ScreenLayout L = make_screen_layout(d, lda_max, 4, nt, cfg->slots);

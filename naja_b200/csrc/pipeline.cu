@@ -152,7 +152,7 @@ extern "C" int naja_chr_run_backmapped(const naja_polytope* P, const naja_chr_pa
   if (!v_dev && ((st = bv0.alloc(chunk_rows * n * velt, stream)) || (st = bv1.alloc(chunk_rows * n * velt, stream))))
     return st;
   if (tc) {
-    // (a shorter last chunk never takes more rows at a time than a whole one)
+    // (a chunk of chains is mapped at one go, so its rows bound the scratch)
     const size_t yb = backmap_tc_operand_bytes(static_cast<long long>(chunk_rows), d, mode);
     const size_t tb = backmap_tc_operand_bytes(n, d, mode);
     if ((st = bTh.alloc(tb, stream)) || (st = bTl.alloc(tb, stream)) || (st = bYh.alloc(yb, stream)) ||
