@@ -41,3 +41,27 @@ def test_final_slack(cuda, m, precision):
     P = Polytope(*_polytope(m, 5, seed=m))
     a, b = _run(P, precision=precision), _run(P, precision=precision, max_slots=2)
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("kind", ["plain", "subnormal", "huge", "small_bounds"])
+@pytest.mark.parametrize("m", [150, 901, 2500, 3300])
+def test_every_row_divided(cuda, m, kind, precision):
+    """Two rows of zero width take half of the steps off the short cut, at each
+    of the smaller thread counts; with entries whose quotients are not normal
+    numbers, and with all slacks small."""
+    A, b = _polytope(m, 6, seed=m)
+    row = np.concatenate([np.ones(3), np.zeros(3)])
+    A, b = np.vstack([A, row, -row]), np.concatenate([b, [0.0, 0.0]])
+    if kind == "subnormal":
+        A[5::7] *= 1e-40
+    elif kind == "huge":
+        A[5::7] *= 1e16
+        b[5::7] *= 1e-20
+    elif kind == "small_bounds":
+        b = b * 1e-18
+    S = Polytope(A, b)
+    kw = dict(seed=5, pair_prob=0.4, resync_interval=11, precision=precision)
+    got = S.run(np.zeros(6), 20, 3, 3, out_dtype="f64", sparse="dense", **kw)
+    S.check()
+    assert np.array_equal(got, O.chr_run(A, b, np.zeros(6), 20, 3, 3, **kw), equal_nan=True)
