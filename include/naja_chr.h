@@ -173,7 +173,8 @@ typedef struct naja_batch_config {
 int naja_chr_run_batched(int nmodels, const naja_polytope* const* models, const naja_chr_params* params,
                          const double* const* X0s, int ldx, void* const* samples, double* const* X_finals,
                          unsigned long long seed_stride, const naja_batch_config* config, void* stream);
-/* Resident chains per SM that `config` allows for these models (0 if none). */
+/* Resident chains per SM that `config` allows for these models (0 if none),
+ * in a run of Philox streams without k-sparse steps (others may differ). */
 int naja_batch_occupancy(int nmodels, const naja_polytope* const* models, const naja_batch_config* config,
                          int* ctas_per_sm);
 /* The same batched launch captured once into a CUDA graph (*graph receives
