@@ -78,7 +78,7 @@ template <int NT, int R, bool SS>
 int batch_launch_one(const ChrArgs& base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                      const BatchConfig& cfg, cudaStream_t stream) {
   auto kern = chr_batched_kernel<NT, R, SS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern, align_up(sizeof(ChrArgs), 128));
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   int occ = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NT + 32, cfg.smem);
@@ -96,7 +96,7 @@ int batch_launch_one(const ChrArgs& base, const ModelDesc* models, const int* im
 template <int NT, int R, bool SS>
 int batch_occupancy_one(const BatchConfig& cfg, int* out) {
   auto kern = chr_batched_kernel<NT, R, SS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern, align_up(sizeof(ChrArgs), 128));
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, kern, NT + 32, cfg.smem);
   return e == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;

@@ -839,7 +839,8 @@ __global__ void __launch_bounds__(NW * 32 + 64, NW >= 8 ? 2 : (NW == 4 ? 4 : 6))
 template <int NW, int E>
 int batch_columns_one(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                       const BatchConfig& cfg, cudaStream_t stream, int* occ_out) {
-  return batch_run(chr_batched_columns_kernel<NW, E>, NW * 32 + 64, cfg, nitems, occ_out, [&](auto kern, int grid) {
+  return batch_run(chr_batched_columns_kernel<NW, E>, NW * 32 + 64, align_up(sizeof(ChrArgs) + sizeof(SpArgs), 128), cfg,
+                   nitems, occ_out, [&](auto kern, int grid) {
     const ColLayout L = make_col_layout(base->d, cfg.lda_max, sizeof(float), NW, E, cfg.slots);
     kern<<<grid, NW * 32 + 64, cfg.smem, stream>>>(*base, L, models, im, ic, nitems);
   });

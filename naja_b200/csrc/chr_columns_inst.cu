@@ -11,7 +11,7 @@ namespace {
 template <class Real, int NW, int E, bool RES>
 int launch_columns(const ChrArgs& a, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream) {
   auto kern = chr_columns_kernel<Real, NW, E, RES>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   const ColLayout L = make_col_layout(a.d, a.m, sizeof(Real), NW, E, cfg.resident ? 0 : cfg.slots);
   kern<<<nchains, NW * 32 + 64, cfg.smem, stream>>>(a, sp, L);

@@ -544,8 +544,7 @@ int chr_batch_slack(const ModelDesc* models, int nmodels, int nchains, int m_max
   const dim3 grid((m_max + 127) / 128, nmodels);
   auto launch = [&](auto kern, int cg) {
     const size_t smem = static_cast<size_t>(cg) * d * sizeof(double);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-      return NAJA_ERR_CUDA;
+    if (allow_smem(kern) != cudaSuccess) return NAJA_ERR_CUDA;
     kern<<<grid, 128, smem, stream>>>(models, nchains, d);
     return cudaGetLastError() == cudaSuccess ? NAJA_OK : NAJA_ERR_CUDA;
   };

@@ -87,6 +87,14 @@ struct RedEntry {
 };
 
 constexpr size_t kSmemBudget = 227 * 1024;
+
+// Lets a kernel ask for all the shared memory that a plan may give it beside
+// its `fixed` static bytes: one limit per kernel whatever the launch, so that
+// threads that launch it with different layouts do not undo each other's.
+template <class Kern>
+cudaError_t allow_smem(Kern kern, size_t fixed = 0) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBudget - fixed));
+}
 constexpr int kMaxSlots = 8;
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1189,7 +1197,7 @@ __global__ void __launch_bounds__(NT + 32, 1)
 template <class Real, int NT, int R>
 int launch_one_cluster(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream) {
   auto kern = chr_cluster_kernel<Real, NT, R>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern, 1024);
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   const Layout L = make_layout(a.d, cfg.slice_lda, sizeof(Real), NT, cfg.slots);
   cudaLaunchConfig_t lc = {};
@@ -1216,7 +1224,7 @@ int launch_one(const ChrArgs& a, int nchains, const ChrLaunchConfig& cfg, cudaSt
   if (cfg.cluster > 1) return NAJA_ERR_UNSUPPORTED;
   if (UNI && a.m % kStandaloneV<Real> != 0) return NAJA_ERR_UNSUPPORTED;
   auto kern = chr_kernel<Real, NT, R, UNI>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   const Layout L = make_layout(a.d, a.lda, sizeof(Real), NT, cfg.slots);
   kern<<<nchains, NT + 32, cfg.smem, stream>>>(a, L);

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, 1)
 template <class Real, int NW, bool SCAT>
 int launch_sparse(const ChrArgs& a, const SpArgs& sp, int nchains, const ChrLaunchConfig& cfg, cudaStream_t stream) {
   auto kern = chr_sparse_kernel<Real, NW, SCAT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   const Layout L =
       make_sparse_layout(a.d, a.m, sizeof(Real), sizeof(SpEntry<Real>), cfg.max_col, NW, cfg.slots, SCAT);
@@ -679,7 +679,7 @@ template <int NW>
 int batch_sparse_one(const ChrArgs* base, const ModelDesc* models, const int* im, const int* ic, int nitems,
                      const BatchConfig& cfg, cudaStream_t stream, int* occ_out) {
   auto kern = chr_batched_sparse_kernel<NW>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem));
+  cudaError_t e = allow_smem(kern, align_up(sizeof(ChrArgs) + sizeof(SpArgs), 128));
   if (e != cudaSuccess) return NAJA_ERR_CUDA;
   int occ = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NW * 32 + 32, cfg.smem);

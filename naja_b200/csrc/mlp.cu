@@ -311,9 +311,12 @@ cudaError_t gemm_launch(const CUtensorMap& mA, const CUtensorMap& mB, GemmArgs a
   a.tiles = static_cast<long long>((a.M + kTileM - 1) / kTileM) * a.tiles_n;
   // the MMA reads 128 rows of A from the last stage on: the blocks behind the
   // ring are more than the 64 rows that may be missing there
-  const size_t smem = a.stages * stage + 1024 + 512 + 4 * kStagePad * sizeof(float);
+  constexpr size_t beside = 1024 + 512 + 4 * kStagePad * sizeof(float);
+  const size_t smem = a.stages * stage + beside;
   const cudaError_t e =
-      cudaFuncSetAttribute(gemm_bf16_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      // (one limit whatever the product: threads with different ones do not undo each other's)
+      cudaFuncSetAttribute(gemm_bf16_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kRingBudget + beside));
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(std::min<long long>(sms, a.tiles));
   gemm_bf16_kernel<TN><<<grid, kThreads, smem, stream>>>(mA, mB, a);

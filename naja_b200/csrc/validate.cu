@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kEssThreads) ess_kernel(const float* __restric
 constexpr int kRhatThreads = 1024;
 constexpr int kRhatWarps = kRhatThreads / 32;
 constexpr int kRhatLoads = 8;
+constexpr size_t kRhatMeans = 128 * 1024;  // bytes kept for the means
 __global__ void __launch_bounds__(kRhatThreads) rhat_kernel(const float* __restrict__ s, long N, int dim, int nchains,
                                                             int layout, int lg_group, int subs, bool keep,
                                                             double* __restrict__ rhat) {
@@ -324,7 +325,9 @@ extern "C" int naja_validate(const float* samples, long long N, int dim, int nch
   }
   if (ess) {
     const size_t smem = (static_cast<size_t>(spc) + kEssPad) * sizeof(float);
-    cudaFuncSetAttribute(ess_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    // (one limit whatever the series: threads with different ones do not undo each other's)
+    cudaFuncSetAttribute(ess_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>((kEssMaxSeries + kEssPad) * sizeof(float)));
     ess_kernel<<<dim * nchains, kEssThreads, smem, stream>>>(static_cast<const float*>(ds), static_cast<long>(N), dim,
                                                              nchains, layout, de);
   }
@@ -335,9 +338,9 @@ extern "C" int naja_validate(const float* samples, long long N, int dim, int nch
     while (lg > 0 && (1 << (lg - 1)) >= dim) --lg;
     while (subs < kRhatWarps && subs < 2 * nchains) subs *= 2;
     const size_t means = (static_cast<size_t>(2) * nchains * sizeof(double)) << lg;
-    const bool keep = means <= 128 * 1024;
+    const bool keep = means <= kRhatMeans;
     const size_t smem = keep ? means : 0;
-    cudaFuncSetAttribute(rhat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaFuncSetAttribute(rhat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRhatMeans));
     rhat_kernel<<<static_cast<unsigned>((dim + (1 << lg) - 1) >> lg), kRhatThreads, smem, stream>>>(
         static_cast<const float*>(ds), static_cast<long>(N), dim, nchains, layout, lg, subs, keep, dr);
   }
